@@ -803,7 +803,7 @@ class TransformerLM:
 
     def _lm_head(self, h, normed: bool = False):
         hn = h if normed else ops.rmsnorm(h, self.final_norm_w, self.eps, self.norm_w_offset)
-        logits = ops.gemm(hn, self.lm_head_w, epi="f32")
+        logits = ops.gemm(hn, self.lm_head_w, epi="f32", w_ready=True)
         scale = getattr(self, "logit_scale", 1.0)
         if scale != 1.0:
             logits = logits * scale
@@ -887,7 +887,7 @@ class TransformerLM:
     def _row_parallel(self, a, w, bias, residual, next_norm_w):
         """residual += a . w^T (summed over TP ranks); returns rmsnorm(residual) * next_norm_w (or None)."""
         if self.tp.size == 1:
-            ops.gemm(a, w, epi="residual", residual=residual, bias=bias, out=residual)
+            ops.gemm(a, w, epi="residual", residual=residual, bias=bias, out=residual, w_ready=True)
             if next_norm_w is None:
                 return None
             return ops.rmsnorm(residual, next_norm_w, self.eps, self.norm_w_offset)
@@ -915,7 +915,7 @@ class TransformerLM:
 
     def _attention_block(self, i, lw, h, st: InferState):
         D, hq, hkv = self.head_dim, self.hq, self.hkv
-        qkv = ops.gemm(h, lw.qkv_w, bias=lw.qkv_b)
+        qkv = ops.gemm(h, lw.qkv_w, bias=lw.qkv_b, w_ready=True)
         kv_layer = self._kv_layer(i)
         cos, sin, rope_rows = self._rope_inputs(st, i)
         ops.rope_kv_scatter_(qkv, kv_layer, cos, sin, rope_rows, st.mem_index, hq, hkv, D,
@@ -935,9 +935,9 @@ class TransformerLM:
 
     def _dense_ffn(self, lw, h):
         if lw.gate_up_fused:
-            act = ops.gemm(h, lw.gate_up_w, epi="gated_" + self.act)
+            act = ops.gemm(h, lw.gate_up_w, epi="gated_" + self.act, w_ready=True)
         else:
-            act = ops.gated_act(ops.gemm(h, lw.gate_up_w), self.act)
+            act = ops.gated_act(ops.gemm(h, lw.gate_up_w, w_ready=True), self.act)
         return "rowpar", act, lw.down_w
 
     def _ffn_block(self, i, lw, h, st):

@@ -226,13 +226,13 @@ class DeepseekV2LM(TransformerLM):
         T = h.shape[0]
         hq, nope, rope, kvl = self.hq, self.nope, self.rope_d, self.kv_lora
         if self.q_lora:
-            qkv_a = ops.gemm(h, lw.qkv_a_w)                       # [T, q_lora + kv_lora + rope]
+            qkv_a = ops.gemm(h, lw.qkv_a_w, w_ready=True)                       # [T, q_lora + kv_lora + rope]
             q_a = ops.rmsnorm(qkv_a[:, : self.q_lora], lw.q_a_norm, self.eps)
             kv_a = qkv_a[:, self.q_lora:]
-            q = ops.gemm(q_a, lw.q_b_w)                           # [T, hq * (nope + rope)]
+            q = ops.gemm(q_a, lw.q_b_w, w_ready=True)                           # [T, hq * (nope + rope)]
         else:
-            q = ops.gemm(h, lw.q_b_w)
-            kv_a = ops.gemm(h, lw.kv_a_w)
+            q = ops.gemm(h, lw.q_b_w, w_ready=True)
+            kv_a = ops.gemm(h, lw.kv_a_w, w_ready=True)
         q3 = q.view(T, hq, nope + rope)
         kv_layer = self._kv_layer(i)                      # [slots, 1, kvl + rope]
         ops.mla_rope_kv_scatter_(q3, kv_a, kv_layer, lw.kv_a_norm, self.cos, self.sin, st.position_ids, st.mem_index,

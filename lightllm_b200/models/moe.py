@@ -155,7 +155,7 @@ def moe_ffn(model, lw, h, mc: MoEConfig, layer: int = -1, st=None):
     """Returns the per-rank partial sum [T, H] of routed (+ shared) experts, written where the TP reduction
     wants it."""
     T = h.shape[0]
-    logits = ops.gemm(h, lw.router_w, epi="f32")
+    logits = ops.gemm(h, lw.router_w, epi="f32", w_ready=True)
     if mc.scoring == "softmax" and mc.n_group <= 1:
         ids, w = moe_ops.topk_softmax(logits, mc.top_k, mc.renorm, mc.routed_scale)
     else:

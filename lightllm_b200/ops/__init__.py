@@ -221,8 +221,25 @@ def _tuned_bn(M: int, N: int, K: int, epi: str) -> int:
     return _autotuner.gemm_lookup(M, N, K, epi)
 
 
+# Up to this many tokens a plain weight goes through csrc/gemm_stream.cu (weights as the MMA's M side).
+STREAM_MAX_M = 128
+_STREAM_EPIS = ("store", "residual", "gated_silu", "f32", "gated_gelu", "relu2")
+
+
+def _stream_rule(M: int, N: int, K: int, epi: str, bias) -> bool:
+    """Up to 64 tokens always.  With more of them a CTA stages as many token bytes as weight bytes, and the 256-column kernels are
+    ahead (B200, us per call in a chain, here / there: [4096, 14336] 42 / 35, [6144, 4096] 22 / 18, and [128256, 4096] 210 / 196,
+    whose tiles read the tokens once per wave), except where those leave SMs idle: a weight whose 128-row tiles fill one and a half to
+    two CTAs per SM without shares of K ([28672, 4096] 51 / 93), or a small one ([5120, 2048] 12 / 17, [2048, 4096] 14 / 17)."""
+    if not (0 < M <= STREAM_MAX_M and N >= 1024 and K >= 1024 and N % 8 == 0 and epi in _STREAM_EPIS):
+        return False
+    if bias is not None and epi.startswith("gated"):
+        return False
+    return M <= 64 or 148 * 128 < N <= 2 * 148 * 128 or N * K <= 12 << 20
+
+
 def gemm(a, w, epi: str = "store", residual=None, bias=None, out=None, bn: int = 0, stream_k: int = 0,
-         out_scale: float = 1.0, x=None, dyt=None, clamp=None, softcap: float = 0.0):
+         out_scale: float = 1.0, x=None, dyt=None, clamp=None, softcap: float = 0.0, w_ready: bool = False):
     """C = A . W^T on the tcgen05 tensor cores.  a [M, K], w [N, K] (checkpoint layout).  fp32 operands run on the
     CUDA cores in fp32 (`csrc/gemm_f32.cu`).
 
@@ -233,6 +250,8 @@ def gemm(a, w, epi: str = "store", residual=None, bias=None, out=None, bn: int =
     x += post(A . W^T) in place and C = next(x) | "gated_clamp": interleaved as the other gated forms, with
     clamp = (alpha, limit): g = min(g, limit), u = clamp(u, -limit, limit), C = (u + 1) g sigmoid(alpha g).
     stream_k: 0 whole tiles per CTA (default: fastest on every measured shape), 1 stream-K, -1 heuristic.
+    w_ready: w was not written by the kernel queued just before this call (a layer's weights): with few tokens its first
+    tiles are then fetched while that kernel still runs.
     """
     if type(w).__name__ == "Fp8Weight":  # block-scaled e4m3 weight: quantise the activations, fp8 tensor cores
         from . import fp8
@@ -261,9 +280,20 @@ def gemm(a, w, epi: str = "store", residual=None, bias=None, out=None, bn: int =
         return res
     M, K = a.shape
     N = w.shape[0]
+    if stream_k == 0 and not isinstance(w, TiledWeight) and (4000 <= bn < 4100 or bn == 0 and _stream_rule(M, N, K, epi, bias)):
+        if bn == 0:   # a stored variant of this kernel is a number of K shares; other variants were tuned before it was there
+            bn = _tuned_bn(M, N, K, epi) if bias is None else 0
+        return _gemm_stream(a, w, epi, residual, bias, out, bn - 4000 if 4000 <= bn < 4100 else 0, w_ready)
+    return _gemm_tiles(a, w, epi, residual, bias, out, bn, stream_k)
+
+
+def _gemm_tiles(a, w, epi="store", residual=None, bias=None, out=None, bn=0, stream_k=0):
+    M, K = a.shape
+    N = w.shape[0]
     tiled = isinstance(w, TiledWeight)
     if bn == 0 and stream_k == 0 and M <= 256 and bias is None and not tiled:  # a tuned variant, if one is stored
         bn = _tuned_bn(M, N, K, epi)
+        bn = 0 if bn >= 4000 else bn
     ldw = (-2 if w.swizzled else -1) if tiled else w.stride(0)
     if tiled:
         w = w.data
@@ -281,6 +311,23 @@ def gemm(a, w, epi: str = "store", residual=None, bias=None, out=None, bn: int =
                                   c_int(bn), c_int(stream_k), ptr(skp), i64(skp.numel() if skp is not None else 0),
                                   ptr(skc), c_int(skc.numel() if skc is not None else 0),
                                   ptr(gemm_status(a.device)), stream()), "gemm_bf16")
+    _count()
+    return out
+
+
+def _gemm_stream(a, w, epi, residual, bias, out, splits, w_ready):
+    M, K = a.shape
+    N = w.shape[0]
+    assert w.shape[1] == K and w.stride(1) == 1 and a.stride(1) == 1
+    if out is None:
+        out = torch.empty((M, N // 2 if epi.startswith("gated") else N), dtype=torch.float32 if epi == "f32" else a.dtype,
+                          device=a.device)
+    if epi == "residual":
+        assert residual.shape == out.shape and residual.stride(0) == out.stride(0)
+    check(kernels().llb_gemm_stream(ptr(a), i64(a.stride(0)), ptr(w), i64(w.stride(0)), ptr(out), i64(out.stride(0)),
+                                    ptr(residual), ptr(bias), c_int(M), c_int(N), c_int(K), c_int(EPI_CODES[epi]),
+                                    c_int(splits), f32(1.0), f32(0.0), c_int(int(w_ready)), ptr(gemm_status(a.device)),
+                                    stream()), "gemm_stream")
     _count()
     return out
 

@@ -162,9 +162,10 @@ def tune(candidates: Sequence[dict], bench: Callable[[dict], float], group=None)
 GEMM_KERNEL = "gemm_bf16"
 # `bn` selectors understood by ops.gemm: 0 automatic plan, 64 / 128 / 256 one-CTA tiles, 512 CTA-pair tiles,
 # 1000 + 10 * accumulators + splits cluster kernel (+ 100: 128-column tiles), 2000 + splits one-CTA tiles and
-# 3000 + splits CTA-pair tiles with K split through the L2 workspace (x000: as many splits as fit)
+# 3000 + splits CTA-pair tiles with K split through the L2 workspace (x000: as many splits as fit), 4000 + splits the few-token
+# kernel (the only variants looked at where `ops._stream_rule` holds)
 GEMM_CANDIDATES = [{"bn": b} for b in (0, 64, 128, 256, 512, 1011, 1012, 1014, 1021, 1111, 1112,
-                                       2000, 2002, 2004, 3000, 3001, 3002, 3004)]
+                                       2000, 2002, 2004, 3000, 3001, 3002, 3004, 4001, 4002, 4003, 4004, 4006, 4008)]
 
 
 def gemm_static_key(N: int, K: int, epi: str) -> str:
