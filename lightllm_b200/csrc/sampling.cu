@@ -1,9 +1,9 @@
 // Token sampling over fp32 logits [B, V]: penalties, temperature, softmax, top-k / top-p
-// filtering and the draw itself, one CTA per request, no sort.
+// filtering and the draw itself, one cluster of CTAs per request, no sort.
 //
 //   * the top-k / top-p cut is found by bisection on the logit value: the kept set is
 //     S(tau) = {i : x_i >= tau}; the largest tau with |S| >= k or mass(S) >= p is the
-//     tighter of the two filters (each pass is one sweep over the row, served by L2);
+//     tighter of the two filters (each pass is one sweep over the row, which the cluster keeps in shared memory);
 //   * the draw is an exponential race: argmax_i p_i / E_i with E_i ~ Exp(1) from a
 //     counter-based generator keyed by (seed, step, i), so a request with a fixed seed
 //     reproduces its stream whatever batch it lands in;
@@ -187,6 +187,160 @@ sample_kernel(const T* __restrict__ logits, int64_t stride, int V, const float* 
   }
 }
 
+// The same sampler with the row shared out over a cluster of 8 CTAs that keep their slices (inv_t * logit) in shared memory.
+// The one-CTA form above sweeps the row up to 27 times through L2 with a single SM, 4 bytes per thread and load: 708 us for 24 rows
+// of 128256 logits.  Here the row is read once and a sweep is 32 shared-memory reads per thread and one cluster barrier.
+//   * a sum (count and mass above `mid`, or an arg-max) is pushed to all peers and added up in rank order by everyone, so the CTAs
+//     take the same branches; two buffers in turn make one barrier per sum enough
+//   * the bisection stops early once at most one logit lies in [lo, hi): the set kept for lo can no longer change
+constexpr int kRowCtas = 8;
+constexpr int kRowThreads = 512;      // two CTAs per SM: 37 rows at once
+constexpr int kSliceMax = 48 * 1024;  // floats of a slice (192 KB)
+
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void push_f2(uint32_t addr, float a, float b) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void row_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// sum of (a, b) over the cluster, the same bits in every thread.  sh: a float2 per warp; box: [2][kRowCtas] float2 filled by the peers
+__device__ __forceinline__ float2 row_sum2(float a, float b, float2* sh, float2* box, int& turn, int rank) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  a = warp_sum(a), b = warp_sum(b);
+  if (lane == 0) sh[w] = make_float2(a, b);
+  __syncthreads();
+  float2* mine = box + turn * kRowCtas;
+  if (w == 0) {
+    const float2 t = lane < kRowThreads / 32 ? sh[lane] : make_float2(0.f, 0.f);
+    a = warp_sum(t.x), b = warp_sum(t.y);
+    if (lane < kRowCtas) push_f2(peer_addr(smem_u32(mine + rank), lane), a, b);
+  }
+  row_barrier();
+  turn ^= 1;
+  float2 r = mine[0];
+#pragma unroll
+  for (int i = 1; i < kRowCtas; ++i) r.x += mine[i].x, r.y += mine[i].y;
+  return r;
+}
+__device__ __forceinline__ ArgMax row_argmax(ArgMax a, float2* sh, float2* box, int& turn, int rank) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  auto warp_best = [](ArgMax v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      v = better(v, ArgMax{__shfl_xor_sync(0xffffffffu, v.v, o), __shfl_xor_sync(0xffffffffu, v.i, o)});
+    return v;
+  };
+  a = warp_best(a);
+  if (lane == 0) sh[w] = make_float2(a.v, __int_as_float(a.i));
+  __syncthreads();
+  float2* mine = box + turn * kRowCtas;
+  if (w == 0) {
+    a = warp_best(lane < kRowThreads / 32 ? ArgMax{sh[lane].x, __float_as_int(sh[lane].y)} : ArgMax{-INFINITY, 0x7fffffff});
+    if (lane < kRowCtas) push_f2(peer_addr(smem_u32(mine + rank), lane), a.v, __int_as_float(a.i));
+  }
+  row_barrier();
+  turn ^= 1;
+  ArgMax r{mine[0].x, __float_as_int(mine[0].y)};
+#pragma unroll
+  for (int i = 1; i < kRowCtas; ++i) r = better(r, ArgMax{mine[i].x, __float_as_int(mine[i].y)});
+  return r;
+}
+
+template <typename T>
+__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads, 2)
+sample_row_kernel(const T* __restrict__ logits, int64_t stride, int V, int slice, const float* __restrict__ temperature,
+                  const float* __restrict__ top_p, const int* __restrict__ top_k, const uint64_t* __restrict__ seeds,
+                  const int64_t* __restrict__ steps, int64_t* __restrict__ out_ids, float* __restrict__ out_logprob) {
+  extern __shared__ float xs[];
+  __shared__ float2 sh[kRowThreads / 32];
+  __shared__ __align__(16) float2 box[2 * kRowCtas];
+  const int b = blockIdx.y, rank = blockIdx.x;
+  const T* row = logits + (int64_t)b * stride;
+  const int i0 = min(V, rank * slice), n = min(V, i0 + slice) - i0;
+  const int k = top_k ? top_k[b] : 1;
+  const bool greedy = (k == 1);
+  float temp = temperature ? temperature[b] : 1.f;
+  if (greedy || temp < 1e-5f) temp = 1.f;
+  const float inv_t = 1.f / temp;
+  int turn = 0;
+  row_barrier();  // a peer's shared memory may be written once that peer runs
+
+  ArgMax best{-INFINITY, 0x7fffffff};
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n; i += kRowThreads) {
+    const float x = ld_logit(row, i0 + i) * inv_t;
+    xs[i] = x;  // read again by this thread alone
+    best = better(best, ArgMax{x, i0 + i});
+  }
+  best = row_argmax(best, sh, box, turn, rank);
+  const float xmax = best.v;
+  float z = 0.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += kRowThreads) z += __expf(xs[i] - xmax);
+  z = row_sum2(z, 0.f, sh, box, turn, rank).x;
+  const float logz = __logf(z);
+
+  if (greedy || (temperature && temperature[b] < 1e-5f)) {
+    if (rank == 0 && threadIdx.x == 0) {
+      out_ids[b] = best.i;
+      if (out_logprob) out_logprob[b] = -logz;
+    }
+    return;
+  }
+
+  const float p_lim = top_p ? top_p[b] : 1.f;
+  const bool use_p = p_lim < 1.f;
+  const bool use_k = k > 0 && k < V;
+  float tau = -INFINITY;  // keep everything
+  if (use_p || use_k) {
+    float lo = xmax - 30.f, hi = xmax;  // predicate true at lo (or the tail below it is < 1e-13 of the mass)
+    float cnt_lo = INFINITY, cnt_hi = 0.f;  // logits >= lo and >= hi: bounds until the first probe on that side
+    const float need_mass = p_lim * z;
+    for (int it = 0; it < 24 && cnt_lo - cnt_hi > 1.f; ++it) {
+      const float mid = 0.5f * (lo + hi);
+      float cnt = 0.f, mass = 0.f;
+#pragma unroll 4
+      for (int i = threadIdx.x; i < n; i += kRowThreads) {
+        const float x = xs[i];
+        if (x >= mid) {
+          cnt += 1.f;
+          mass += __expf(x - xmax);
+        }
+      }
+      const float2 s = row_sum2(cnt, mass, sh, box, turn, rank);
+      const bool ok = (use_k && s.x >= (float)k) || (use_p && s.y >= need_mass);
+      if (ok)
+        lo = mid, cnt_lo = s.x;
+      else
+        hi = mid, cnt_hi = s.x;
+    }
+    tau = lo;
+  }
+
+  const uint64_t seed = seeds ? seeds[b] : 0x1234ull + b;
+  const uint64_t step = steps ? (uint64_t)steps[b] : 0ull;
+  ArgMax pick{-INFINITY, 0x7fffffff};
+  for (int i = threadIdx.x; i < n; i += kRowThreads) {
+    const float x = xs[i];
+    if (x >= tau) {
+      const float u = uniform01(seed, step, (uint32_t)(i0 + i));
+      pick = better(pick, ArgMax{x - __logf(-__logf(u)), i0 + i});
+    }
+  }
+  pick = row_argmax(pick, sh, box, turn, rank);
+  if (rank == 0 && threadIdx.x == 0) {
+    const int id = pick.i == 0x7fffffff ? best.i : pick.i;
+    out_ids[b] = id;
+    if (out_logprob) out_logprob[b] = ld_logit(row, id) * inv_t - xmax - logz;
+  }
+}
+
 // log-softmax value of given token ids (prompt_logprobs / chosen-token logprob): out[b] = log p(ids[b])
 template <typename T>
 __global__ void __launch_bounds__(1024)
@@ -219,21 +373,42 @@ LLB_EXPORT int llb_apply_penalty(float* logits, int64_t stride, const float* pre
   return LLB_OK;
 }
 
-// dtype: 0 = fp32 logits, 1 = bf16 logits
+namespace {
+template <typename T>
+int launch_sample(const void* logits, int64_t stride, int B, int V, const float* temperature, const float* top_p,
+                  const int* top_k, const uint64_t* seeds, const int64_t* steps, int64_t* out_ids, float* out_logprob,
+                  cudaStream_t st) {
+  const int slice = cdiv(V, kRowCtas);
+  if (V < 4096 || slice > kSliceMax || B > 65535) {
+    sample_kernel<T><<<B, 1024, 0, st>>>((const T*)logits, stride, V, temperature, top_p, top_k, seeds, steps, out_ids,
+                                         out_logprob);
+    LLB_LAUNCH_CHECK();
+    return LLB_OK;
+  }
+  static DeviceOnce configured;
+  if (!configured.done()) {
+    cudaError_t e = cudaFuncSetAttribute(sample_row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSliceMax * 4);
+    if (e != cudaSuccess) return (int)e;
+    configured.set();
+  }
+  sample_row_kernel<T><<<dim3(kRowCtas, B), kRowThreads, slice * 4, st>>>((const T*)logits, stride, V, slice, temperature, top_p,
+                                                                          top_k, seeds, steps, out_ids, out_logprob);
+  LLB_LAUNCH_CHECK();
+  return LLB_OK;
+}
+}  // namespace
+
+// dtype: 0 = fp32 logits, 1 = bf16 logits.  Rows of 4096 logits and more (up to what 8 CTAs hold) go to the cluster kernel; below
+// that its barriers cost more than the sweeps of one CTA.
 LLB_EXPORT int llb_sample(const void* logits, int dtype, int64_t stride, int B, int V, const float* temperature,
                           const float* top_p, const int* top_k, const uint64_t* seeds, const int64_t* steps,
                           int64_t* out_ids, float* out_logprob, cudaStream_t st) {
   if (B <= 0) return LLB_OK;
   if (dtype == 0)
-    sample_kernel<float><<<B, 1024, 0, st>>>((const float*)logits, stride, V, temperature, top_p, top_k, seeds, steps,
-                                             out_ids, out_logprob);
-  else if (dtype == 1)
-    sample_kernel<bf16><<<B, 1024, 0, st>>>((const bf16*)logits, stride, V, temperature, top_p, top_k, seeds, steps,
-                                            out_ids, out_logprob);
-  else
-    return LLB_ERR_UNSUPPORTED;
-  LLB_LAUNCH_CHECK();
-  return LLB_OK;
+    return launch_sample<float>(logits, stride, B, V, temperature, top_p, top_k, seeds, steps, out_ids, out_logprob, st);
+  if (dtype == 1)
+    return launch_sample<bf16>(logits, stride, B, V, temperature, top_p, top_k, seeds, steps, out_ids, out_logprob, st);
+  return LLB_ERR_UNSUPPORTED;
 }
 
 // ---- all-greedy batches: arg-max + log-probability in two small passes over many CTAs ----
