@@ -3,7 +3,7 @@ layers followed by MoE layers with routed + shared experts, sigmoid (V3) or soft
 top-k routing with an optional score-correction bias, yarn RoPE with mscale.
 
 KV pool row: [c_kv (kv_lora_rank, RMS-normalised) | k_pe (rotated)], one head, replicated over TP ranks.
-Attention runs absorbed (see ops/mla.py): per layer
+Attention runs absorbed (see ops/mla.py), or for longer prompt portions over keys and values formed per head: per layer
     q: x -> q_a_proj -> q_a_layernorm -> q_b_proj (heads sharded over TP)          [or q_proj]
     kv: x -> kv_a_proj_with_mqa (replicated) -> kv_a_layernorm on the latent, RoPE on k_pe -> pool
     q_lat = q_nope . W_UK (per head), MLA attention over the pool, o = o_lat . W_UV^T (per head), o_proj
@@ -172,7 +172,12 @@ class DeepseekV2LM(TransformerLM):
         kvb = kvb.view(h1 - h0, self.nope + self.v_dim, self.kv_lora)
         # W_UK as [h, kv_lora, nope] (q_lat = q_nope . W_UK: contraction over nope), W_UV as [h, v, kv_lora]
         lw.w_uk = self._dev(kvb[:, : self.nope].transpose(1, 2))
-        lw.w_uv = self._dev(kvb[:, self.nope:])
+        if self._can_expand():   # both halves as one K-major matrix: latent row -> [all heads' keys | all heads' values]
+            n = (h1 - h0) * self.nope
+            lw.w_kv = self._dev(torch.cat([kvb[:, : self.nope].reshape(n, -1), kvb[:, self.nope:].reshape(-1, self.kv_lora)]))
+            lw.w_uv = lw.w_kv[n:].view(h1 - h0, self.v_dim, self.kv_lora)
+        else:
+            lw.w_uv = self._dev(kvb[:, self.nope:])
         if self.fp8_compute and (h0 * self.v_dim) % 128 == 0:
             lw.o_w = quant.load_fp8_weight(src, a + "o_proj.weight", 1, h0 * self.v_dim, h1 * self.v_dim).to(self.device)
         else:
@@ -237,10 +242,40 @@ class DeepseekV2LM(TransformerLM):
         kv_layer = self._kv_layer(i)                      # [slots, 1, kvl + rope]
         ops.mla_rope_kv_scatter_(q3, kv_a, kv_layer, lw.kv_a_norm, self.cos, self.sin, st.position_ids, st.mem_index,
                                  nope, rope, kvl, self.eps)
+        groups = self._expanded_groups(st)
+        if groups:
+            return self._expanded_attention(lw, q, kv_layer, st, groups)
         q_lat = mla_ops.gemm_batched(q3[:, :, :nope], lw.w_uk)    # [T, hq, kvl]
         o_lat = self._mla_attend(i, lw, h, q_a if self.q_lora else None, q_lat, q3[:, :, nope:], kv_layer, st)
         o = mla_ops.gemm_batched(o_lat, lw.w_uv)                  # [T, hq, v]
         return o.reshape(T, hq * self.v_dim)
+
+    def _can_expand(self) -> bool:
+        """Prompt passes may form keys and values per head: bf16 on the GPU, the head sizes of the tensor-core kernel, and
+        attention over all cached positions (sparse variants select in the latent space)."""
+        return self.device.type == "cuda" and self.dtype == torch.bfloat16 and self.nope == 128 and self.rope_d == 64 and \
+            self.v_dim in (64, 128) and self.sm_scale > 0 and type(self)._mla_attend is DeepseekV2LM._mla_attend
+
+    def _expanded_groups(self, st):
+        if not st.is_prefill or not self._can_expand():
+            return None
+        if "expanded_groups" not in st.extra:
+            q_len, ready = st.extra["q_len_cpu"].to(torch.int64).cpu(), st.extra["ready_cpu"].to(torch.int64).cpu()
+            groups = mla_ops.expanded_groups(q_len, ready, self.hq * (self.nope + self.v_dim) * 2)
+            st.extra["expanded_groups"] = groups and [(a, b, mla_ops.KeyRange(ready[a:b], q_len[a:b], 0, self.device))
+                                                      for a, b in groups]
+        return st.extra["expanded_groups"]
+
+    def _expanded_attention(self, lw, q, kv_layer, st, groups):
+        """Attention over keys and values formed per head from the latent rows of the pass: [T, hq * v]."""
+        r2t = self.req_manager.req_to_token_indexs
+        out = torch.empty((q.shape[0], self.hq * self.v_dim), dtype=q.dtype, device=q.device)
+        for a, b, kr in groups:
+            c = mla_ops.latent_gather(kv_layer, r2t, st.b_req_idx[a:b], kr)      # [rows, kv_lora + rope]
+            kv = ops.gemm(c[:, : self.kv_lora], lw.w_kv)
+            mla_ops.latent_prefill(q, kv, c, self.kv_lora, self.nope, self.hq, self.head_dim, self.v_dim, st.cu_q[a:b + 1],
+                                   st.b_ready_cache_len[a:b], kr, st.max_q_len, self.sm_scale, out)
+        return out
 
     def _mla_attend(self, i, lw, h, q_a, q_lat, q_pe, kv_layer, st):
         """Absorbed attention over the latent cache: [T, hq, kv_lora].  Sparse variants override this."""

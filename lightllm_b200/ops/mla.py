@@ -252,3 +252,45 @@ def window_prefill(q, kv, H: int, dk: int, dv: int, cu_q, b_ready_len, kr: KeyRa
                                           i64(gate.stride(0) if gate is not None else 0), stream()), "window_prefill_tc")
     _count()
     return out
+
+
+def latent_prefill(q, kv, c, col: int, own: int, H: int, dk: int, dv: int, cu_q, b_ready_len, kr: KeyRange, max_q_len: int, scale,
+                   out):
+    """`window_prefill` without a window, where the last dk - own columns of every head's keys are the columns from `col` on of c
+    [rows, >= col + dk - own]: q [T, >= H * dk], kv [rows, H * own | H * dv], out [T, H * dv] (only the requests of cu_q are written)."""
+    assert q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16 and c.dtype == torch.bfloat16
+    assert q.stride(1) == 1 and kv.is_contiguous() and c.stride(1) == 1 and out.stride(1) == 1 and cu_q.dtype == torch.int32
+    assert kv.shape == (kr.rows, H * (own + dv)) and c.shape[0] == kr.rows and c.shape[1] >= col + dk - own
+    check(kernels().llb_latent_prefill_tc(ptr(q), i64(q.stride(0)), ptr(kv), i64(kv.stride(0)), c_int(kr.rows), ptr(c),
+                                          i64(c.stride(0)), c_int(col), c_int(own), ptr(cu_q), ptr(kr.cu_kv), ptr(kr.kv_start),
+                                          ptr(b_ready_len), ptr(out), i64(out.stride(0)), c_int(cu_q.shape[0] - 1),
+                                          c_int(q.shape[0]), c_int(max_q_len), c_int(H), c_int(dk), c_int(dv), f32(scale),
+                                          stream()), "latent_prefill_tc")
+    _count()
+    return out
+
+
+# Expanded keys and values that a prompt pass holds at a time, in bytes: 32 K positions of 128 heads of 128 + 128
+EXPANDED_BYTES = 2 << 30
+
+
+def expanded_groups(q_len, ready, bytes_per_row: int):
+    """Requests of a prompt pass in runs [first, last) whose expanded keys and values fit EXPANDED_BYTES, or None if the pass is
+    better off in the latent space: one request alone does not fit, or too few new tokens share the expansion.
+
+    q_len, ready: new and cached tokens per request (host).  Per head a position costs 512 x 256 multiply-adds to expand and a
+    (query, key) pair 320 instead of 1088 in the latent space; the expansion and the attention over it run on the tcgen05 tensor
+    cores, the latent kernel on mma.sync at an eighth of that rate or less (B200, 128 heads, 7 requests of 300 to 1500 new tokens behind
+    up to 1000 cached: 22.7 ms a layer there)."""
+    n, seq = q_len.tolist(), (q_len + ready).tolist()
+    pairs = sum(a * (s - a / 2) for a, s in zip(n, seq))
+    if pairs * 1088 * 8 <= sum(seq) * 512 * 256 + pairs * 320 or max(seq) * bytes_per_row > EXPANDED_BYTES:
+        return None
+    groups, first, rows = [], 0, 0
+    for b, s in enumerate(seq):
+        if rows + s > EXPANDED_BYTES // bytes_per_row:
+            groups.append((first, b))
+            first, rows = b, 0
+        rows += s
+    groups.append((first, len(seq)))
+    return groups
