@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128)
 gqa_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const bf16* __restrict__ kv_layer,
                   const int* __restrict__ req_to_token, int64_t r2t_stride, const int* __restrict__ b_req_idx,
                   const int* __restrict__ b_seq_len, bf16* __restrict__ out, int64_t out_stride,
-                  float* __restrict__ part_o, float* __restrict__ part_lse, int Hq, int Hkv, int num_splits,
+                  float* __restrict__ part_o, float* __restrict__ part_lse, int Hq, int Hkv, int num_splits, int B, int shares,
                   float scale_log2, const KeyRule rule, const OutGate gate) {
   pdl_wait();
   constexpr int CH = DK / 8, CHV = DV / 8;             // 16-byte chunks per row
@@ -63,27 +63,35 @@ gqa_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const bf16* __re
   uint8_t* q_smem = smem;                                // 16 x D bf16
   uint8_t* warp_smem = smem + TILE_BYTES + (threadIdx.x >> 5) * WARP_BYTES;
 
-  const int split = blockIdx.x;
   const int G = Hq / Hkv;
   const int gc = (G + 15) >> 4;
   const int kvh = blockIdx.y / gc;
   const int chunk_id = blockIdx.y % gc;
   const int head0 = kvh * G + chunk_id * 16;
   const int nrows = min(16, G - chunk_id * 16);
-  const int b = blockIdx.z;
-  const int req = LLB_CHECK_REQ(b_req_idx[b]);
-  const int L = b_seq_len[b];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
 
+  // tiles [tile0, tile1) of request b's keys -> its partial result number `split` of `count` (tile1 < 0: the split-th of num_splits
+  // equal parts)
+  auto work = [&](int b, int split, int count, int tile0, int tile1) {
+  const int req = LLB_CHECK_REQ(b_req_idx[b]);
+  const int L = b_seq_len[b];
   const int lo = SPLIT_P ? rule.first_seen(L - 1) : 0;
   const int kept = SPLIT_P ? min(rule.keep, lo) : 0;
   const int skip = lo - kept;  // key index n >= kept is position n + skip
-  const int tiles_total = (L - skip + 15) >> 4;
-  const int tiles_per_split = (tiles_total + num_splits - 1) / num_splits;
-  const int s0 = split * tiles_per_split * 16;
-  const int e0 = min(L - skip, s0 + tiles_per_split * 16);
+  if (tile1 < 0) {
+    const int tiles_per_split = (((L - skip + 15) >> 4) + num_splits - 1) / num_splits;
+    tile0 = split * tiles_per_split;
+    tile1 = tile0 + tiles_per_split;
+  }
+  const int s0 = tile0 * 16, e0 = min(L - skip, tile1 * 16);
   auto position = [&](int n) { return !SPLIT_P || n < kept ? n : n + skip; };
+  if (split == 0 && count < num_splits) {  // the request's unused slots: nothing to merge
+    const int spare = num_splits - count;
+    for (int i = threadIdx.x; i < nrows * spare; i += blockDim.x)
+      part_lse[((int64_t)b * Hq + head0 + i / spare) * num_splits + count + i % spare] = -INFINITY;
+  }
 
   if (s0 >= e0) {  // empty split: tell the merge kernel to ignore it
     if (num_splits > 1) {
@@ -335,6 +343,18 @@ gqa_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const bf16* __re
       if (d == 0) part_lse[pi] = den > 0.f ? (M + log2f(den)) * kLn2 : -INFINITY;
     }
   }
+  };
+
+  if (!SPLIT_P && shares > 0) {
+    __shared__ int start[SPLIT_P ? 1 : kMaxShareBatch + 1];
+    const int share = decode_shares(b_seq_len, B, shares, num_splits, start);
+    for_each_share(start, B, share, blockIdx.x, [&](int b, int slot, int count, int tile0, int tile1) {
+      work(b, slot, count, tile0, tile1);
+      __syncthreads();  // the rings and the merge buffers are free again
+    });
+  } else {
+    work(blockIdx.z, blockIdx.x, num_splits, 0, -1);
+  }
 }
 
 template <int D>
@@ -344,17 +364,29 @@ decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ 
   pdl_wait();
   const int bh = blockIdx.x;
   const int b = bh / Hq, h = bh % Hq;
-  const int d = threadIdx.x;
+  const int d = threadIdx.x, lane = threadIdx.x & 31;
+  // every warp weighs the partial results, 32 slots at a time (empty ones: 0), and reads the rows four at a time
   const float* lse = part_lse + (int64_t)bh * num_splits;
   float M = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) M = fmaxf(M, lse[s]);
+  for (int s = lane; s < num_splits; s += 32) M = fmaxf(M, lse[s]);
+  M = warp_max(M);
   float num = 0.f, den = 0.f;
-  if (M != -INFINITY) {
-    for (int s = 0; s < num_splits; ++s) {
-      if (lse[s] == -INFINITY) continue;  // empty split: its partial row was never written
-      float w = __expf(lse[s] - M);
-      num += w * part_o[((int64_t)bh * num_splits + s) * D + d];
-      den += w;
+  for (int s0 = 0; s0 < num_splits; s0 += 32) {
+    const float l = s0 + lane < num_splits ? lse[s0 + lane] : -INFINITY;
+    const float mine = l == -INFINITY ? 0.f : __expf(l - M);
+    den += warp_sum(mine);
+    const float* o = part_o + ((int64_t)bh * num_splits + s0) * D + d;
+    for (uint32_t left = __ballot_sync(0xffffffffu, mine != 0.f); left != 0;) {
+      float w[4], v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int s = left != 0 ? __ffs((int)left) - 1 : -1;
+        left &= left - 1;
+        w[u] = s < 0 ? 0.f : __shfl_sync(0xffffffffu, mine, s);
+        v[u] = s < 0 ? 0.f : o[(int64_t)s * D];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) num += w[u] * v[u];
     }
   }
   out[(int64_t)b * out_stride + (int64_t)h * D + d] = __float2bfloat16(den > 0.f ? num / den * gate_factor<D>(gate, b, h, d) : 0.f);
@@ -559,12 +591,16 @@ int set_smem(K kernel, int bytes) {
 
 // Number of KV splits the decode launcher will use for a batch (the caller sizes the
 // scratch buffers with it): enough CTAs to fill the GPU, at least 256 tokens per split.
+// The most CTAs that work on one request's context (slots of partial results per request; 1: no merge).  With `w` of them for a
+// request of average length the GPU is full (four CTAs per SM wanted); a long one may get 4 w (see decode_shares).  A batch that fills
+// the GPU twice over runs unsplit.
+constexpr int kDecodeCtas = 148 * 4;
 LLB_EXPORT int llb_gqa_decode_num_splits(int B, int Hq, int Hkv, int max_seq_len) {
   int G = Hq / Hkv;
   int ctas = B * Hkv * ((G + 15) / 16);
-  int target = 148 * 4;
-  int want = (target + ctas - 1) / ctas;
-  int cap = (max_seq_len + 255) / 256;
+  if (ctas >= 2 * kDecodeCtas) return 1;
+  int want = 4 * ((kDecodeCtas + ctas - 1) / ctas);
+  int cap = (max_seq_len + 16 * kMinShareTiles - 1) / (16 * kMinShareTiles);
   if (cap < 1) cap = 1;
   int s = want < cap ? want : cap;
   if (s < 1) s = 1;
@@ -579,7 +615,10 @@ static int launch_decode(const void* q, int64_t q_stride, const void* kv_layer, 
                          const OutGate& gate, cudaStream_t st) {
   constexpr int STAGES = decode_stages<DK, DV>();
   const int G = Hq / Hkv;
-  const dim3 grid(num_splits, Hkv * ((G + 15) / 16), B);
+  const int groups = Hkv * ((G + 15) / 16);
+  // Shares of equal length, one wave of two CTAs per SM (100 KB of rings each)
+  const int shares = !SPLIT_P && num_splits > 1 && B <= kMaxShareBatch ? (kDecodeCtas / 2 > groups ? kDecodeCtas / 2 / groups : 1) : 0;
+  const dim3 grid = shares > 0 ? dim3(shares, groups, 1) : dim3(num_splits, groups, B);
   static DeviceOnce configured;
   if (!configured.done()) {
     int rc = set_smem(gqa_decode_kernel<DK, DV, STAGES, SPLIT_P>, decode_smem_bytes<DK, DV>());
@@ -588,7 +627,7 @@ static int launch_decode(const void* q, int64_t q_stride, const void* kv_layer, 
   }
   launch_pdl(gqa_decode_kernel<DK, DV, STAGES, SPLIT_P>, grid, dim3(128), decode_smem_bytes<DK, DV>(), st, (const bf16*)q,
              q_stride, (const bf16*)kv_layer, req_to_token, r2t_stride, b_req_idx, b_seq_len, (bf16*)out, out_stride, part_o,
-             part_lse, Hq, Hkv, num_splits, sm_scale * kLog2e, rule, gate);
+             part_lse, Hq, Hkv, num_splits, B, shares, sm_scale * kLog2e, rule, gate);
   LLB_LAUNCH_CHECK();
   if (num_splits > 1) {
     launch_pdl(decode_merge_kernel<DV>, dim3(B * Hq), dim3(DV), 0, st, (const float*)part_o, (const float*)part_lse,

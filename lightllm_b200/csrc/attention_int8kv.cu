@@ -493,7 +493,7 @@ gqa_decode_q8_regs_kernel(const bf16* __restrict__ q, int64_t q_stride, const in
                           const int* __restrict__ req_to_token, int64_t r2t_stride, const int* __restrict__ b_req_idx,
                           const int* __restrict__ b_seq_len, bf16* __restrict__ out, int64_t out_stride,
                           float* __restrict__ part_o, float* __restrict__ part_lse, int Hq, int Hkv, int num_splits,
-                          float scale_log2_in, const float* __restrict__ head_scales) {
+                          int B, int shares, float scale_log2_in, const float* __restrict__ head_scales) {
   pdl_wait();
   constexpr int D = 128;
   constexpr int ROW = FP8 ? D : D + kPad;          // bytes of a row in the pool
@@ -501,25 +501,32 @@ gqa_decode_q8_regs_kernel(const bf16* __restrict__ q, int64_t q_stride, const in
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t* warp_smem = smem + (threadIdx.x >> 5) * kRegWarpBytes;
 
-  const int split = blockIdx.x;
   const int G = Hq / Hkv;
   const int gc = (G + 15) >> 4;
   const int kvh = blockIdx.y / gc;
   const int chunk_id = blockIdx.y % gc;
   const int head0 = kvh * G + chunk_id * 16;
   const int nrows = min(16, G - chunk_id * 16);
-  const int b = blockIdx.z;
-  const int req = b_req_idx[b];
-  const int L = b_seq_len[b];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
   const float scale_log2 = FP8 ? scale_log2_in * head_scales[kvh] : scale_log2_in;
   const float out_scale = FP8 ? head_scales[Hkv + kvh] : 1.f;
 
-  const int tiles_total = (L + 15) >> 4;
-  const int tiles_per_split = (tiles_total + num_splits - 1) / num_splits;
-  const int s0 = split * tiles_per_split * 16;
-  const int e0 = min(L, s0 + tiles_per_split * 16);
+  // as in gqa_decode_kernel (attention.cu)
+  auto work = [&](int b, int split, int count, int tile0, int tile1) {
+  const int req = b_req_idx[b];
+  const int L = b_seq_len[b];
+  if (tile1 < 0) {
+    const int tiles_per_split = (((L + 15) >> 4) + num_splits - 1) / num_splits;
+    tile0 = split * tiles_per_split;
+    tile1 = tile0 + tiles_per_split;
+  }
+  const int s0 = tile0 * 16, e0 = min(L, tile1 * 16);
+  if (split == 0 && count < num_splits) {  // the request's unused slots: nothing to merge
+    const int spare = num_splits - count;
+    for (int i = threadIdx.x; i < nrows * spare; i += blockDim.x)
+      part_lse[((int64_t)b * Hq + head0 + i / spare) * num_splits + count + i % spare] = -INFINITY;
+  }
 
   if (s0 >= e0) {
     if (num_splits > 1) {
@@ -761,6 +768,18 @@ gqa_decode_q8_regs_kernel(const bf16* __restrict__ q, int64_t q_stride, const in
       if (d == 0) part_lse[pi] = den > 0.f ? (M + log2f(den)) * kLn2 : -INFINITY;
     }
   }
+  };
+
+  if (shares > 0) {
+    __shared__ int start[kMaxShareBatch + 1];
+    const int share = decode_shares(b_seq_len, B, shares, num_splits, start);
+    for_each_share(start, B, share, blockIdx.x, [&](int b, int slot, int count, int tile0, int tile1) {
+      work(b, slot, count, tile0, tile1);
+      __syncthreads();  // the rings and the merge buffers are free again
+    });
+  } else {
+    work(blockIdx.z, blockIdx.x, num_splits, 0, -1);
+  }
 }
 
 template <int D>
@@ -770,17 +789,29 @@ decode_merge_int8_kernel(const float* __restrict__ part_o, const float* __restri
   pdl_wait();
   const int bh = blockIdx.x;
   const int b = bh / Hq, h = bh % Hq;
-  const int d = threadIdx.x;
+  const int d = threadIdx.x, lane = threadIdx.x & 31;
+  // every warp weighs the partial results, 32 slots at a time (empty ones: 0), and reads the rows four at a time
   const float* lse = part_lse + (int64_t)bh * num_splits;
   float M = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) M = fmaxf(M, lse[s]);
+  for (int s = lane; s < num_splits; s += 32) M = fmaxf(M, lse[s]);
+  M = warp_max(M);
   float num = 0.f, den = 0.f;
-  if (M != -INFINITY) {
-    for (int s = 0; s < num_splits; ++s) {
-      if (lse[s] == -INFINITY) continue;
-      float w = __expf(lse[s] - M);
-      num += w * part_o[((int64_t)bh * num_splits + s) * D + d];
-      den += w;
+  for (int s0 = 0; s0 < num_splits; s0 += 32) {
+    const float l = s0 + lane < num_splits ? lse[s0 + lane] : -INFINITY;
+    const float mine = l == -INFINITY ? 0.f : __expf(l - M);
+    den += warp_sum(mine);
+    const float* o = part_o + ((int64_t)bh * num_splits + s0) * D + d;
+    for (uint32_t left = __ballot_sync(0xffffffffu, mine != 0.f); left != 0;) {
+      float w[4], v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int s = left != 0 ? __ffs((int)left) - 1 : -1;
+        left &= left - 1;
+        w[u] = s < 0 ? 0.f : __shfl_sync(0xffffffffu, mine, s);
+        v[u] = s < 0 ? 0.f : o[(int64_t)s * D];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) num += w[u] * v[u];
     }
   }
   out[(int64_t)b * out_stride + (int64_t)h * D + d] = __float2bfloat16(den > 0.f ? num / den : 0.f);
@@ -851,9 +882,12 @@ int launch_decode8(const void* q, int64_t q_stride, const void* kv_layer, const 
       if (e != cudaSuccess) return (int)e;
       configured.set();  
     }
-    launch_pdl(gqa_decode_q8_regs_kernel<FP8>, grid, dim3(128), kRegSmemBytes, st, (const bf16*)q, q_stride,
-               (const int8_t*)kv_layer, req_to_token, r2t_stride, b_req_idx, b_seq_len, (bf16*)out, out_stride,
-               part_o, part_lse, Hq, Hkv, num_splits, sl2, head_scales);
+    // shares of equal length, one wave of three CTAs per SM (registers, 72 KB of rings each)
+    const int groups = Hkv * ((G + 15) / 16), ctas = 148 * 3;
+    const int shares = num_splits > 1 && B <= kMaxShareBatch ? (ctas > groups ? ctas / groups : 1) : 0;
+    launch_pdl(gqa_decode_q8_regs_kernel<FP8>, shares > 0 ? dim3(shares, groups, 1) : grid, dim3(128), kRegSmemBytes, st,
+               (const bf16*)q, q_stride, (const int8_t*)kv_layer, req_to_token, r2t_stride, b_req_idx, b_seq_len, (bf16*)out,
+               out_stride, part_o, part_lse, Hq, Hkv, num_splits, B, shares, sl2, head_scales);
     LLB_LAUNCH_CHECK();
     if (num_splits > 1) {
       launch_pdl(decode_merge_int8_kernel<128>, dim3(B * Hq), dim3(128), 0, st, (const float*)part_o,

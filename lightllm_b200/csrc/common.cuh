@@ -206,6 +206,64 @@ struct KeyRule {
     return chunk > 0 ? p - p % chunk : 0;
   }
 };
+// Work of a decode step whose contexts are cut into shares of equal length over the whole batch: the 16-token tiles of all requests
+// lie back to back, CTA `cta` of `ctas` takes tiles [cta * share, (cta + 1) * share), which may end one request and begin others.
+// With the same number of shares per request instead, ragged contexts make the longest one's shares last several times the mean,
+// and a grid of more CTAs than fit at once ends in a wave that is nearly empty.  A share has at least kMinShareTiles, and no
+// request touches more than `cap` CTAs (the slots of its partial results).  start [B + 1] (shared): first tile of each request; every
+// request has at least one.  Every CTA does the same prefix sum over the lengths (B loads, served by L2); 128 threads, all take part.
+constexpr int kMinShareTiles = 8;
+constexpr int kMaxShareBatch = 592;
+__device__ __forceinline__ int decode_shares(const int* __restrict__ seq_len, int B, int ctas, int cap, int* start) {
+  __shared__ int sums[4], longest[4];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int each = (B + 127) / 128, b0 = t * each < B ? t * each : B, b1 = b0 + each < B ? b0 + each : B;
+  int sum = 0, most = 0;
+  for (int b = b0; b < b1; ++b) {
+    const int len = seq_len[b], tiles = len > 0 ? (len + 15) >> 4 : 1;
+    start[b + 1] = tiles;
+    sum += tiles;
+    most = tiles > most ? tiles : most;
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  int upto = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += v;
+  }
+  if (lane == 31) sums[w] = upto, longest[w] = most;
+  __syncthreads();
+  for (int i = 0; i < w; ++i) upto += sums[i];
+  int at = upto - sum;
+  if (t == 0) start[0] = 0;
+  for (int b = b0; b < b1; ++b) {
+    at += start[b + 1];
+    start[b + 1] = at;
+  }
+  __syncthreads();
+  const int total = sums[0] + sums[1] + sums[2] + sums[3];
+  most = max(max(longest[0], longest[1]), max(longest[2], longest[3]));
+  return max(max((total + ctas - 1) / ctas, kMinShareTiles), (most + cap - 2) / (cap - 1));
+}
+// Runs body(b, slot, slots, first tile, end tile) for every request that CTA `cta` works on; slot: which of the request's `slots` CTAs.
+template <typename Body>
+__device__ __forceinline__ void for_each_share(const int* start, int B, int share, int cta, Body body) {
+  int u = cta * share;
+  const int end = min(u + share, start[B]);
+  if (u >= end) return;
+  int b = 0;
+  for (int hi = B - 1; b < hi;) {
+    const int mid = (b + hi + 1) >> 1;
+    if (start[mid] <= u) b = mid; else hi = mid - 1;
+  }
+  for (; u < end; ++b) {
+    const int s = start[b], e = start[b + 1], first = s / share;
+    body(b, cta - first, (e - 1) / share - first + 1, u - s, min(end, e) - s);
+    u = e;
+  }
+}
+
 // Sigmoid gate on attention outputs: one value per row and head, or (elem) one per row and output element, at gate[row * stride].
 struct OutGate {
   const void* gate;  // or null

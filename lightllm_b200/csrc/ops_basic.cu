@@ -5,6 +5,7 @@
 // GEMM also exist as GEMM epilogues (see gemm_tcgen05.cu), the standalone forms
 // here serve the first/last layer and the non-fused paths.
 #include "common.cuh"
+#include <cuda_fp8.h>
 
 using namespace llb;
 LLB_DEBUG_BOUNDS_STORAGE(ops_basic)
@@ -146,9 +147,13 @@ LLB_EXPORT int llb_gated_act(void* out, const void* x, int T, int I, int act, cu
 //   pos        [T] int32, slot [T] int32 (destination slot of each new token)
 // A group of D/8 consecutive lanes owns one head (each lane one 16-byte vector); the
 // rotation partner's values come by warp shuffle, so every lane writes only its own vector.
+// KV = 1, 2: quantised pools (rows of D int8 + fp32 scale + 12 bytes, and rows of D e4m3 with static scales per head): the bf16 values
+// that the plain form stores are quantised on the way, with the arithmetic of the separate store (kv_quant_store_int8_kernel; x /
+// scale to e4m3), which cost two more launches (int8) or eight of generic elementwise kernels (fp8, 20 us a layer).
 // ---------------------------------------------------------------------------------------
-template <int LANES_PER_HEAD>
-__global__ void __launch_bounds__(256) rope_kv_scatter_kernel(bf16* __restrict__ qkv, bf16* __restrict__ kv_layer,
+template <int LANES_PER_HEAD, int KV>
+__global__ void __launch_bounds__(256) rope_kv_scatter_kernel(bf16* __restrict__ qkv, void* __restrict__ kv_pool,
+                                                              const float* __restrict__ head_scales,
                                                               const float* __restrict__ cos_t,
                                                               const float* __restrict__ sin_t,
                                                               const int* __restrict__ pos, const int* __restrict__ slot,
@@ -211,25 +216,56 @@ __global__ void __launch_bounds__(256) rope_kv_scatter_kernel(bf16* __restrict__
         x[k] = lower ? (x[k] * c - y[k] * sn) : (x[k] * c + y[k] * sn);
       }
     }
-    if (!valid) continue;
     bf16x8 o = pack8(x);
+    float amax = 0.f;
+    if (KV != 0) {
+      unpack8(o, x);  // what is stored in bf16
+      if (KV == 1) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(x[k]));
+#pragma unroll
+        for (int u = LANES_PER_HEAD / 2; u > 0; u >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, u));
+      }
+    }
+    if (!valid) continue;
     if (kind == 0) {
       reinterpret_cast<bf16x8*>(row + (int64_t)head * D)[v] = o;
+      continue;
+    }
+    const int h = head - Hq;  // 0..2*Hkv-1 : K heads then V heads, the pool's order
+    const int64_t at = (int64_t)s * (2 * Hkv) + h;
+    if (KV == 0) {
+      reinterpret_cast<bf16x8*>((bf16*)kv_pool + at * D)[v] = o;
     } else {
-      int h = head - Hq;  // 0..2*Hkv-1 : K heads then V heads, the pool's order
-      reinterpret_cast<bf16x8*>(kv_layer + ((int64_t)s * (2 * Hkv) + h) * D)[v] = o;
+      const float scale = KV == 2 ? head_scales[h] : (amax > 0.f ? amax / 127.f : 1.f);
+      uint32_t w[2] = {0u, 0u};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        uint32_t byte;
+        if (KV == 1) {
+          const float q = fminf(fmaxf(rintf(x[k] / scale), -127.f), 127.f);
+          byte = (uint32_t)(uint8_t)(int8_t)q;
+        } else {
+          byte = (uint32_t)__nv_cvt_float_to_fp8(x[k] / scale, __NV_SATFINITE, __NV_E4M3);
+        }
+        w[k >> 2] |= byte << (8 * (k & 3));
+      }
+      uint8_t* dst = (uint8_t*)kv_pool + at * (KV == 1 ? D + 16 : D);
+      *reinterpret_cast<uint2*>(dst + v * 8) = make_uint2(w[0], w[1]);
+      if (KV == 1 && v == 0) *reinterpret_cast<float*>(dst + D) = scale;
     }
   }
 }
 
-LLB_EXPORT int llb_rope_kv_scatter(void* qkv, void* kv_layer, const float* cos_t, const float* sin_t, const int* pos,
-                                   const int* slot, const void* q_norm_w, const void* k_norm_w, float norm_eps,
-                                   float norm_w_offset, int T, int Hq, int Hkv, int D, int rot_dim, int64_t qkv_stride,
-                                   cudaStream_t st) {
+namespace {
+template <int KV>
+int launch_rope(void* qkv, void* kv_layer, const float* head_scales, const float* cos_t, const float* sin_t, const int* pos,
+                const int* slot, const void* q_norm_w, const void* k_norm_w, float norm_eps, float norm_w_offset, int T, int Hq,
+                int Hkv, int D, int rot_dim, int64_t qkv_stride, cudaStream_t st) {
   if (T <= 0) return LLB_OK;
   if (rot_dim % 16 != 0 || rot_dim > D) return LLB_ERR_UNSUPPORTED;
-#define LAUNCH_ROPE(L)                                                                                              \
-  launch_pdl(rope_kv_scatter_kernel<L>, dim3(T), dim3(256), 0, st, (bf16*)qkv, (bf16*)kv_layer, cos_t, sin_t, pos,  \
+#define LAUNCH_ROPE(L)                                                                                                   \
+  launch_pdl(rope_kv_scatter_kernel<L, KV>, dim3(T), dim3(256), 0, st, (bf16*)qkv, kv_layer, head_scales, cos_t, sin_t, pos, \
              slot, (const bf16*)q_norm_w, (const bf16*)k_norm_w, norm_eps, norm_w_offset, Hq, Hkv, rot_dim, qkv_stride)
   if (D == 128)
     LAUNCH_ROPE(16);
@@ -242,6 +278,27 @@ LLB_EXPORT int llb_rope_kv_scatter(void* qkv, void* kv_layer, const float* cos_t
 #undef LAUNCH_ROPE
   LLB_LAUNCH_CHECK();
   return LLB_OK;
+}
+}  // namespace
+
+LLB_EXPORT int llb_rope_kv_scatter(void* qkv, void* kv_layer, const float* cos_t, const float* sin_t, const int* pos,
+                                   const int* slot, const void* q_norm_w, const void* k_norm_w, float norm_eps,
+                                   float norm_w_offset, int T, int Hq, int Hkv, int D, int rot_dim, int64_t qkv_stride,
+                                   cudaStream_t st) {
+  return launch_rope<0>(qkv, kv_layer, nullptr, cos_t, sin_t, pos, slot, q_norm_w, k_norm_w, norm_eps, norm_w_offset, T, Hq, Hkv,
+                        D, rot_dim, qkv_stride, st);
+}
+
+// The same into a quantised pool: fp8 = 0 int8 rows [slots, 2*Hkv, D + 16], 1 e4m3 rows [slots, 2*Hkv, D] with head_scales [2*Hkv].
+LLB_EXPORT int llb_rope_kv_scatter_q8(void* qkv, void* kv_layer, int fp8, const float* head_scales, const float* cos_t,
+                                      const float* sin_t, const int* pos, const int* slot, const void* q_norm_w,
+                                      const void* k_norm_w, float norm_eps, float norm_w_offset, int T, int Hq, int Hkv, int D,
+                                      int rot_dim, int64_t qkv_stride, cudaStream_t st) {
+  if (((uintptr_t)kv_layer & 15) || (fp8 && head_scales == nullptr)) return LLB_ERR_BAD_ARG;
+  return fp8 ? launch_rope<2>(qkv, kv_layer, head_scales, cos_t, sin_t, pos, slot, q_norm_w, k_norm_w, norm_eps, norm_w_offset, T,
+                              Hq, Hkv, D, rot_dim, qkv_stride, st)
+             : launch_rope<1>(qkv, kv_layer, nullptr, cos_t, sin_t, pos, slot, q_norm_w, k_norm_w, norm_eps, norm_w_offset, T, Hq,
+                              Hkv, D, rot_dim, qkv_stride, st);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -4,7 +4,8 @@ A (slot, head) row of the pool is `D` int8 values followed by one fp32 scale and
 scale = max|x| / 127 over the row), so a token's row is an opaque byte string for everything that moves KV around.
 `Int8KVLayer` wraps one layer's slice of the pool; the attention ops accept it wherever they take a bf16 slice:
 
-* new K / V rows are rotated into a scratch tensor and quantised into their slots (`quant_store_`);
+* new K / V rows are rotated and quantised into their slots in one kernel (other head sizes and `Int4KVLayer`: through a scratch
+  tensor and `quant_store_`);
 * decode attention reads the int8 rows directly (`csrc/attention_int8kv.cu`);
 * prefill (and the generic-head-size kernel) runs on a bf16 copy of the rows the batch refers to, gathered and
   widened once per layer, with a request table that points into that copy.
@@ -207,14 +208,31 @@ def quant_store_(layer, src: torch.Tensor, slot: torch.Tensor) -> None:
     _count()
 
 
-def rope_kv_scatter_(qkv, layer, cos, sin, pos, slot, Hq, Hkv, D, *rest, **kw):
-    """The rotary / norm / scatter op with a quantised destination: K and V go through a scratch tensor."""
-    from . import rope_kv_scatter_ as plain
+def rope_kv_scatter_(qkv, layer, cos, sin, pos, slot, Hq, Hkv, D, rot_dim=None, q_norm_w=None, k_norm_w=None, norm_eps=1e-6,
+                     norm_w_offset=0.0):
+    """The rotary / norm / scatter op with a quantised destination.  On the GPU, 8-bit rows of the usual head sizes are quantised by the
+    same kernel; else K and V go through a scratch tensor."""
+    from . import _count, _req_bf16, c_int, check, f32, i64, kernels, ptr, rope_kv_scatter_ as plain, stream
 
+    rest = (rot_dim, q_norm_w, k_norm_w, norm_eps, norm_w_offset)
+    rot = D if rot_dim is None else rot_dim
+    fp8 = isinstance(layer, Fp8KVLayer)
+    if qkv.is_cuda and (fp8 or isinstance(layer, Int8KVLayer)) and D in (64, 128, 256) and rot % 16 == 0 and rot <= D:
+        _req_bf16(qkv, q_norm_w, k_norm_w)
+        assert qkv.stride(-1) == 1 and layer.data.is_contiguous() and layer.data.shape[1] == 2 * Hkv and layer.head_dim == D
+        assert pos.dtype == torch.int32 and slot.dtype == torch.int32
+        assert rot == 0 or (cos.dtype == torch.float32 and cos.shape[-1] == rot // 2)
+        assert not fp8 or (layer.scales.dtype == torch.float32 and layer.scales.is_contiguous())
+        check(kernels().llb_rope_kv_scatter_q8(ptr(qkv), ptr(layer.data), c_int(int(fp8)), ptr(layer.scales if fp8 else None),
+                                               ptr(cos), ptr(sin), ptr(pos), ptr(slot), ptr(q_norm_w), ptr(k_norm_w),
+                                               f32(norm_eps), f32(norm_w_offset), c_int(qkv.shape[0]), c_int(Hq), c_int(Hkv),
+                                               c_int(D), c_int(rot), i64(qkv.stride(0)), stream()), "rope_kv_scatter_q8")
+        _count()
+        return qkv
     T = qkv.shape[0]
     tmp = torch.empty((T, 2 * Hkv, D), dtype=qkv.dtype, device=qkv.device)
     ident = torch.arange(T, dtype=torch.int32, device=qkv.device)
-    plain(qkv, tmp, cos, sin, pos, ident, Hq, Hkv, D, *rest, **kw)
+    plain(qkv, tmp, cos, sin, pos, ident, Hq, Hkv, D, *rest)
     quant_store_(layer, tmp, slot)
     return qkv
 
