@@ -263,12 +263,13 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 __global__ void __launch_bounds__(256) quant_fp8_group128_kernel(const bf16* __restrict__ x, int64_t ldx,
                                                                  uint8_t* __restrict__ q, int64_t ldq,
                                                                  float* __restrict__ scale, int64_t scale_ld, int M,
-                                                                 int K, int k_groups) {
+                                                                 int K, int k_groups, const int* __restrict__ pair) {
   pdl_wait();
   const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= (int64_t)M * k_groups) return;
   const int row = (int)(w / k_groups), g = (int)(w - (int64_t)row * k_groups);
+  if (pair != nullptr && pair[row] < 0) return;  // a padding row of the expert-sorted order
   const int col = g * 128 + lane * 4;
   float v[4] = {0.f, 0.f, 0.f, 0.f};
   if (col + 4 <= K) {
@@ -500,16 +501,20 @@ int cached_tmap8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t col
 }  // namespace
 
 // x [M, K] bf16 (row pitch ldx) -> q [M, K] e4m3 (row pitch ldq bytes, a multiple of 16) and
-// scale [ceil(K / 128), scale_ld] fp32 (scale_ld >= M).
-LLB_EXPORT int llb_quant_fp8_group128(const void* x, int64_t ldx, void* q, int64_t ldq, float* scale,
-                                      int64_t scale_ld, int M, int K, cudaStream_t st) {
+// scale [ceil(K / 128), scale_ld] fp32 (scale_ld >= M).  pair [M] or null: rows with a negative entry are left out.
+LLB_EXPORT int llb_quant_fp8_group128_rows(const void* x, int64_t ldx, void* q, int64_t ldq, float* scale, int64_t scale_ld, int M,
+                                           int K, const int* pair, cudaStream_t st) {
   if (M <= 0 || K <= 0) return LLB_OK;
   if ((ldx % 4) || (ldq % 4) || ((uintptr_t)x & 7) || ((uintptr_t)q & 3) || scale_ld < M) return LLB_ERR_BAD_ARG;
   const int kg = cdiv(K, 128);
   const int64_t warps = (int64_t)M * kg;
   cudaError_t e = launch_pdl(quant_fp8_group128_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st,
-                             (const bf16*)x, ldx, (uint8_t*)q, ldq, scale, scale_ld, M, K, kg);
+                             (const bf16*)x, ldx, (uint8_t*)q, ldq, scale, scale_ld, M, K, kg, pair);
   return e == cudaSuccess ? LLB_OK : (int)e;
+}
+LLB_EXPORT int llb_quant_fp8_group128(const void* x, int64_t ldx, void* q, int64_t ldq, float* scale,
+                                      int64_t scale_ld, int M, int K, cudaStream_t st) {
+  return llb_quant_fp8_group128_rows(x, ldx, q, ldq, scale, scale_ld, M, K, nullptr, st);
 }
 
 // C[M, N] (bf16; N / 2 columns for the gated epilogue) from e4m3 A [M, K] (pitch lda bytes) and W [n_rows_total, K]

@@ -128,7 +128,7 @@ def _check_sources(specs):
 @register_model("katarax")
 class KataraxLM(StreamLM):
     model_type = "katarax"
-    native_units = ("attention", "attention_generic", "attention_tc", "gemm_f32", "gemm_tcgen05", "latent_attn", "moe",
+    native_units = ("attention", "attention_generic", "attention_tc", "gemm_f32", "gemm_stream", "gemm_tcgen05", "latent_attn", "moe",
                     "ops_basic", "rms_stream", "sampling", "window_prefill_tc")
 
     # ------------------------------------------------------------------ config

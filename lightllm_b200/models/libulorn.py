@@ -112,7 +112,7 @@ class LayerSpec:
 @register_model("libulorn")
 class LibulornLM(RecurrentStateMixin, StreamLM):
     model_type = "libulorn"
-    native_units = ("attention", "attention_generic", "attention_tc", "gemm_f32", "gemm_tcgen05", "moe", "ops_basic",
+    native_units = ("attention", "attention_generic", "attention_tc", "gemm_f32", "gemm_stream", "gemm_tcgen05", "moe", "ops_basic",
                     "recurrent", "rms_stream", "sampling")
 
     # ------------------------------------------------------------------ config

@@ -129,7 +129,7 @@ class Run:
 @register_model("silupel")
 class SilupelLM(RecurrentStateMixin, StreamLM):
     model_type = "silupel"
-    native_units = ("attention", "attention_generic", "attention_tc", "gated_scan", "gemm_f32", "gemm_tcgen05", "latent_attn",
+    native_units = ("attention", "attention_generic", "attention_tc", "gated_scan", "gemm_f32", "gemm_stream", "gemm_tcgen05", "latent_attn",
                     "norm_shift", "ops_basic", "sampling", "window_prefill_tc")
 
     # ------------------------------------------------------------------ config

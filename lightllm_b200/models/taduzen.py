@@ -80,7 +80,7 @@ class LayerSpec:
 @register_model("taduzen")
 class TaduzenLM(StreamLM):
     model_type = "taduzen"
-    native_units = ("dyt", "gemm_f32", "gemm_tcgen05", "latent_attn", "moe", "ops_basic", "sampling",
+    native_units = ("dyt", "gemm_f32", "gemm_stream", "gemm_tcgen05", "latent_attn", "moe", "ops_basic", "sampling",
                     "window_prefill_tc")
 
     # ------------------------------------------------------------------ config

@@ -131,16 +131,27 @@ class Fp8Experts:
         return self.w.nbytes()
 
 
-def quant_act(x: torch.Tensor):
-    """bf16 [M, K] -> (e4m3 [M, K], scale [ceil(K/128), M]).  CUDA: one warp per (token, group)."""
+STREAM_MAX_M = 128
+
+
+def _stream_rule(M: int, N: int) -> bool:
+    """The few-token kernel (csrc/gemm_stream.cu).  Above 64 tokens it reads every weight tile twice, which pays only for narrow
+    outputs, whose tiles would leave SMs idle otherwise (B200, us, here / there: 128 tokens [4096, 7168] 21 / 29, [8192, 8192] 39 / 35,
+    [57344, 8192] 188 / 104; 64 tokens [8192, 28672] 69 / 107, [8192, 8192] 23 / 34, [57344, 8192] 99 / 100)."""
+    return M <= (STREAM_MAX_M if N <= 4096 else min(64, STREAM_MAX_M))
+
+
+def quant_act(x: torch.Tensor, pair=None):
+    """bf16 [M, K] -> (e4m3 [M, K], scale [ceil(K/128), M]).  CUDA: one warp per (token, group).  pair [M] int32 (or None): rows
+    with a negative entry may be left undefined."""
     if not x.is_cuda:
         return quant_act_reference(x)
     assert x.dtype == torch.bfloat16 and x.stride(1) == 1
     M, K = x.shape
     q = torch.empty((M, K), dtype=FP8, device=x.device)
     s = torch.empty((_cdiv(K, GROUP), M), dtype=torch.float32, device=x.device)
-    check(kernels().llb_quant_fp8_group128(ptr(x), i64(x.stride(0)), ptr(q), i64(K), ptr(s), i64(M), ctypes.c_int(M),
-                                           ctypes.c_int(K), stream()), "quant_fp8_group128")
+    check(kernels().llb_quant_fp8_group128_rows(ptr(x), i64(x.stride(0)), ptr(q), i64(K), ptr(s), i64(M), ctypes.c_int(M),
+                                                ctypes.c_int(K), ptr(pair), stream()), "quant_fp8_group128")
     _count()
     return q, s
 
@@ -156,9 +167,11 @@ def _epilogue_reference(acc, epi, residual):
 
 
 def gemm_fp8_quantized(xq, xs, w: Fp8Weight, epi: str = "store", residual=None, out=None,
-                       mblock_expert: Optional[torch.Tensor] = None, n_per_expert: Optional[int] = None):
+                       mblock_expert: Optional[torch.Tensor] = None, n_per_expert: Optional[int] = None,
+                       w_ready: bool = False):
     """C = (xq * xs) . (w.q * w.scale)^T.  Grouped mode (mblock_expert given): w stacks the experts, every
-    128-row block i of xq multiplies with expert mblock_expert[i] (-1: skipped, output rows undefined)."""
+    128-row block i of xq multiplies with expert mblock_expert[i] (-1: skipped, output rows undefined).  w_ready as in
+    `ops.gemm`."""
     M, K = xq.shape
     N = n_per_expert if mblock_expert is not None else w.shape[0]
     n_out = N // 2 if epi == "gated_silu" else N
@@ -184,6 +197,14 @@ def gemm_fp8_quantized(xq, xs, w: Fp8Weight, epi: str = "store", residual=None, 
         out = torch.empty((M, n_out), dtype=torch.bfloat16, device=xq.device)
     if epi == "residual":
         assert residual is not None and residual.shape == out.shape and residual.stride(0) == out.stride(0)
+    if mblock_expert is None and _stream_rule(M, N):
+        check(kernels().llb_gemm_stream_fp8(ptr(xq), i64(xq.stride(0)), ptr(xs), i64(xs.stride(0)), ptr(w.q), i64(K),
+                                            ptr(w.scale), ctypes.c_int(w.ws_rows), ctypes.c_int(w.shape[0]), ptr(out),
+                                            i64(out.stride(0)), ptr(residual), ctypes.c_int(M), ctypes.c_int(N),
+                                            ctypes.c_int(K), ctypes.c_int(EPI[epi]), ctypes.c_int(int(w_ready)),
+                                            ptr(gemm_status(xq.device)), stream()), "gemm_stream_fp8")
+        _count()
+        return out
     check(kernels().llb_gemm_fp8_block(ptr(xq), i64(xq.stride(0)), ptr(xs), i64(xs.stride(0)), ptr(w.q), i64(K),
                                        ptr(w.scale), ctypes.c_int(w.ws_rows), ctypes.c_int(w.shape[0]), ptr(out),
                                        i64(out.stride(0)), ptr(residual), ctypes.c_int(M), ctypes.c_int(N),
@@ -197,7 +218,8 @@ def gemm_fp8(a, w: Fp8Weight, epi: str = "store", residual=None, bias=None, out=
     """bf16 activations: quantise per token group, then the block-scaled GEMM.  epi "f32" returns fp32."""
     xq, xs = quant_act(a)
     kernel_epi = "store" if epi == "f32" else epi
-    res = gemm_fp8_quantized(xq, xs, w, kernel_epi, residual, out if epi != "f32" else None)
+    res = gemm_fp8_quantized(xq, xs, w, kernel_epi, residual, out if epi != "f32" else None,
+                             w_ready=True)   # the kernel queued just before is the quantisation of the activations
     if bias is not None:
         res += bias
     if epi == "f32":

@@ -187,12 +187,47 @@ def gather_rows(x, lay: MoeLayout):
     return a
 
 
+FEW_TOKENS = 128   # a decode step: every expert has at most one 128-row block
+
+
+def _few_tokens_experts(x, w13, w2, lay, act):
+    """Both expert GEMMs of a pass of at most FEW_TOKENS tokens (`csrc/gemm_stream.cu`): [m_pad, H] in sorted order, rows of padding
+    undefined.  The first one picks its tokens from x itself, so nothing is gathered."""
+    from . import EPI_CODES
+
+    T, H = x.shape
+    E, N13, _ = w13.shape
+    fp8_w = type(w13).__name__ == "Fp8Experts"
+
+    def run(a, scale, w, gather, n, epi, out):
+        f = w.w if fp8_w else None
+        q = f.q if fp8_w else w
+        check(kernels().llb_gemm_stream_experts(
+            ptr(a), i64(a.stride(0)), c_int(int(gather)), ptr(scale), i64(scale.stride(0) if fp8_w else 0), ptr(q),
+            i64(a.shape[1]), ptr(f.scale if fp8_w else None), c_int(f.ws_rows if fp8_w else 0), c_int(E * n), ptr(out),
+            i64(out.stride(0)), ptr(lay.mblock_expert), ptr(lay.sorted_pair), c_int(T), c_int(lay.k), c_int(lay.m_pad), c_int(n),
+            c_int(a.shape[1]), c_int(EPI_CODES[epi]), ptr(gemm_status(a.device)), stream()), "gemm_stream_experts")
+        _count()
+        return out
+
+    h = torch.empty((lay.m_pad, N13 // 2), dtype=x.dtype, device=x.device)
+    y = torch.empty((lay.m_pad, H), dtype=x.dtype, device=x.device)
+    if fp8_w:
+        from . import fp8
+
+        run(*fp8.quant_act(x), w13, True, N13, "gated_" + act, h)
+        return run(*fp8.quant_act(h, lay.sorted_pair), w2, False, H, "store", y)
+    assert w13.is_contiguous() and w2.is_contiguous()
+    run(x, None, w13, True, N13, "gated_" + act, h)
+    return run(h, None, w2, False, H, "store", y)
+
+
 def fused_experts(x, w13, w2, ids, weights, act="silu", e0: int = 0, out=None, accumulate: bool = False,
                   b13=None, b2=None, clamp=SWIGLU_OAI):
     """Routed expert FFN:  out[t] (+)= sum_k w[t,k] * down_e( act(gate_e(x_t)) * up_e(x_t) ),  e = ids[t,k].
 
     w13 [E_local, 2I, H] with gate/up rows interleaved in 32-row blocks, w2 [E_local, H, I].  On CUDA: align
-    -> gather -> grouped GEMM with gated epilogue -> grouped GEMM -> weighted combine (5 launches)."""
+    -> gather -> grouped GEMM with gated epilogue -> grouped GEMM -> weighted combine (5 launches; no gather with few tokens)."""
     fp8_w = type(w13).__name__ == "Fp8Experts"
     if not x.is_cuda:
         if fp8_w:  # CPU: same arithmetic with the de-quantised weights
@@ -210,8 +245,17 @@ def fused_experts(x, w13, w2, ids, weights, act="silu", e0: int = 0, out=None, a
     I = N13 // 2
     k = ids.shape[1]
     lay = moe_align(ids, E_local, e0)
-    a = gather_rows(x, lay)
-    if fp8_w:
+    few = T <= FEW_TOKENS and x.dtype == torch.bfloat16 and x.stride(1) == 1 and b13 is None and b2 is None and \
+        (act == "silu" or act == "gelu" and not fp8_w) and N13 % 64 == 0 and H % 16 == 0 and I % 16 == 0 and \
+        (x.stride(0) * 2) % 16 == 0 and x.data_ptr() % 16 == 0
+    if few:
+        y = _few_tokens_experts(x, w13, w2, lay, act)
+        a = None
+    else:
+        a = gather_rows(x, lay)
+    if few:
+        pass
+    elif fp8_w:
         # block-scaled e4m3 experts: quantise the gathered rows per token group, grouped fp8 GEMM with the SwiGLU
         # epilogue, quantise again, grouped fp8 GEMM (reference: lightllm/common/basemodel/layer_weights/
         # meta_weights/fused_moe/impl/deepgemm_impl.py, the masked / contiguous m_grouped_fp8_gemm_nt path)
@@ -233,7 +277,7 @@ def fused_experts(x, w13, w2, ids, weights, act="silu", e0: int = 0, out=None, a
         check(kernels().llb_moe_bias_act(ptr(h13), ptr(b13), ptr(lay.mblock_expert), ptr(h), c_int(lay.m_pad), c_int(I),
                                          c_int(kind), f32(clamp[0]), f32(clamp[1]), stream()), "moe_bias_act")
         _count()
-    if not fp8_w:
+    if not fp8_w and not few:
         y = gemm_grouped(h, w2, lay.mblock_expert, H, epi="store")
     if b2 is not None:
         check(kernels().llb_moe_add_bias(ptr(y), ptr(b2), ptr(lay.mblock_expert), c_int(lay.m_pad), c_int(H), stream()),
