@@ -4,8 +4,6 @@
 // [T, H * DV] multiplies the result element by element with its sigmoid.
 //
 //   kv [rows, H * DK | H * DV]: request b's keys are rows cu_kv[b] .., position kv_start[b] first
-//   shared part (llb_latent_prefill_tc): kv [rows, H * own | H * DV] and the last DK - own columns of every head's keys are the
-//   same columns of a second matrix (the rotated part of a latent row), which the TMA thread fetches in their place
 //   a query sees its own position and the window - 1 before it  (window 0: all before it)
 //
 // One CTA computes 128 query rows of one (request, head), as in attention_tc.cu: per tile of 128 keys (64 for key sizes above 128) S = Q . K^T into one of
@@ -60,13 +58,11 @@ struct Params {
   int64_t gate_stride;
   int H, window;
   float scale_log2;
-  int own, shared_col;  // key columns of a head in kv; where the shared ones start in their matrix (own == DK: none)
 };
 
 template <int DK, int DV, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
-window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
-                      const __grid_constant__ CUtensorMap tmShared, const Params p) {
+window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV, const Params p) {
   using L = Layout<DK, DV, BN>;
   constexpr int HK = BN / 2;  // keys of a score tile per softmax thread
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -138,16 +134,13 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!mbar_wait(k_empty(stage), par, abort_flag, status, 61)) break;
         mbar_expect_tx(k_full(stage), L::K_BYTES);
 #pragma unroll
-        for (int c = 0; c < DK / 64; ++c) {
-          const bool mine = c * 64 < p.own;
-          tma_load_2d(k_dst + c * L::KV_BLOCK, mine ? &tmKV : &tmShared, k_full(stage),
-                      mine ? h * p.own + c * 64 : p.shared_col + c * 64 - p.own, row0 + j * BN);
-        }
+        for (int c = 0; c < DK / 64; ++c)
+          tma_load_2d(k_dst + c * L::KV_BLOCK, &tmKV, k_full(stage), h * DK + c * 64, row0 + j * BN);
         if (!mbar_wait(v_empty(stage), par, abort_flag, status, 62)) break;
         mbar_expect_tx(v_full(stage), L::V_BYTES);
 #pragma unroll
         for (int c = 0; c < DV / 64; ++c)
-          tma_load_2d(v_dst + c * L::KV_BLOCK, &tmKV, v_full(stage), p.H * p.own + h * DV + c * 64, row0 + j * BN);
+          tma_load_2d(v_dst + c * L::KV_BLOCK, &tmKV, v_full(stage), p.H * DK + h * DV + c * 64, row0 + j * BN);
       }
     }
     __syncwarp();
@@ -357,8 +350,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 }
 
 template <int DK, int DV, int BN>
-int launch(const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ts, const Params& p, int B, int max_q_len,
-           cudaStream_t st) {
+int launch(const CUtensorMap& tq, const CUtensorMap& tkv, const Params& p, int B, int max_q_len, cudaStream_t st) {
   using L = Layout<DK, DV, BN>;
   static_assert(L::BYTES <= 227 * 1024, "shared memory");
   static_assert(8 * 32 * (DV + 16) <= L::OFF_KV, "output staging fits the Q / P buffers");
@@ -370,7 +362,7 @@ int launch(const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ts,
     configured.set();
   }
   const dim3 grid((max_q_len + BM - 1) / BM, p.H, B);
-  window_prefill_kernel<DK, DV, BN><<<grid, THREADS, L::BYTES, st>>>(tq, tkv, ts, p);
+  window_prefill_kernel<DK, DV, BN><<<grid, THREADS, L::BYTES, st>>>(tq, tkv, p);
   LLB_LAUNCH_CHECK();
   return LLB_OK;
 }
@@ -384,43 +376,6 @@ LLB_EXPORT int llb_window_tc_status() {
   return v;
 }
 
-namespace {
-int prefill(const void* q, int64_t q_stride, const void* kv, int64_t kv_stride, int kv_rows, const void* shared,
-            int64_t shared_stride, int shared_col, int own, const int* cu_q, const int* cu_kv, const int* kv_start,
-            const int* b_ready_len, void* out, int64_t out_stride, int B, int T, int max_q_len, int H, int dk, int dv,
-            float sm_scale, int window, const void* gate, int64_t gate_stride, cudaStream_t st) {
-  if (B <= 0 || max_q_len <= 0 || T <= 0) return LLB_OK;
-  if (!(sm_scale > 0.f) || H <= 0 || H > 65535 || B > 65535 || kv_rows <= 0 || window < 0) return LLB_ERR_BAD_ARG;
-  if ((dk != 64 && dk != 128 && dk != 192 && dk != 256) || (dv != 64 && dv != 128)) return LLB_ERR_UNSUPPORTED;
-  if (own <= 0 || own > dk || (own % 64)) return LLB_ERR_UNSUPPORTED;
-  if (own < dk && (shared == nullptr || shared_col < 0 || (shared_col % 8))) return LLB_ERR_BAD_ARG;
-  if (gate != nullptr && ((gate_stride % 8) || ((uintptr_t)gate & 15))) return LLB_ERR_BAD_ARG;
-  const int bn = dk > 128 ? 64 : 128;
-  if ((out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
-  CUtensorMap tq, tkv, ts;
-  int rc = make_tmap_2d(&tq, q, 2, (uint64_t)T, (uint64_t)H * dk, (uint64_t)q_stride, BM, 64);
-  if (rc) return rc;
-  rc = make_tmap_2d(&tkv, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (own + dv), (uint64_t)kv_stride, bn, 64);
-  if (rc) return rc;
-  ts = tkv;
-  if (own < dk) {
-    rc = make_tmap_2d(&ts, shared, 2, (uint64_t)kv_rows, (uint64_t)shared_col + dk - own, (uint64_t)shared_stride, bn, 64);
-    if (rc) return rc;
-  }
-  const Params p{cu_q, cu_kv, kv_start, b_ready_len, (bf16*)out, out_stride, (const bf16*)gate, gate_stride, H, window,
-                 sm_scale * kLog2e, own, shared_col};
-#define LLB_WINDOW(DK, BN)                                                                                                \
-  if (dk == DK)                                                                                                           \
-    return dv == 64 ? launch<DK, 64, BN>(tq, tkv, ts, p, B, max_q_len, st) : launch<DK, 128, BN>(tq, tkv, ts, p, B, max_q_len, st);
-  LLB_WINDOW(64, 128)
-  LLB_WINDOW(128, 128)
-  LLB_WINDOW(192, 64)
-  LLB_WINDOW(256, 64)
-#undef LLB_WINDOW
-  return LLB_ERR_UNSUPPORTED;
-}
-}  // namespace
-
 // q [T, >= H * DK] bf16 (row pitch q_stride), kv [kv_rows, H * (DK + DV)] (pitch kv_stride), out [T, H * DV]; gate
 // [T, >= H * DV] or null: out *= sigmoid(gate).
 LLB_EXPORT int llb_window_prefill_tc(const void* q, int64_t q_stride, const void* kv, int64_t kv_stride, int kv_rows,
@@ -428,17 +383,26 @@ LLB_EXPORT int llb_window_prefill_tc(const void* q, int64_t q_stride, const void
                                      void* out, int64_t out_stride, int B, int T, int max_q_len, int H, int dk, int dv,
                                      float sm_scale, int window, const void* gate, int64_t gate_stride,
                                      cudaStream_t st) {
-  return prefill(q, q_stride, kv, kv_stride, kv_rows, nullptr, 0, 0, dk, cu_q, cu_kv, kv_start, b_ready_len, out, out_stride, B, T,
-                 max_q_len, H, dk, dv, sm_scale, window, gate, gate_stride, st);
-}
-
-// Keys of head h: columns h * own .. of kv [kv_rows, H * own | H * dv], then columns shared_col .. of `shared` [kv_rows, >= shared_col
-// + dk - own] (pitch shared_stride), the same for all heads.  Causal, no window.
-LLB_EXPORT int llb_latent_prefill_tc(const void* q, int64_t q_stride, const void* kv, int64_t kv_stride, int kv_rows,
-                                     const void* shared, int64_t shared_stride, int shared_col, int own, const int* cu_q,
-                                     const int* cu_kv, const int* kv_start, const int* b_ready_len, void* out,
-                                     int64_t out_stride, int B, int T, int max_q_len, int H, int dk, int dv, float sm_scale,
-                                     cudaStream_t st) {
-  return prefill(q, q_stride, kv, kv_stride, kv_rows, shared, shared_stride, shared_col, own, cu_q, cu_kv, kv_start, b_ready_len,
-                 out, out_stride, B, T, max_q_len, H, dk, dv, sm_scale, 0, nullptr, 0, st);
+  if (B <= 0 || max_q_len <= 0 || T <= 0) return LLB_OK;
+  if (!(sm_scale > 0.f) || H <= 0 || H > 65535 || B > 65535 || kv_rows <= 0 || window < 0) return LLB_ERR_BAD_ARG;
+  if ((dk != 64 && dk != 128 && dk != 192 && dk != 256) || (dv != 64 && dv != 128)) return LLB_ERR_UNSUPPORTED;
+  if (gate != nullptr && ((gate_stride % 8) || ((uintptr_t)gate & 15))) return LLB_ERR_BAD_ARG;
+  const int bn = dk > 128 ? 64 : 128;
+  if ((out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
+  CUtensorMap tq, tkv;
+  int rc = make_tmap_2d(&tq, q, 2, (uint64_t)T, (uint64_t)H * dk, (uint64_t)q_stride, BM, 64);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tkv, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (dk + dv), (uint64_t)kv_stride, bn, 64);
+  if (rc) return rc;
+  const Params p{cu_q, cu_kv, kv_start, b_ready_len, (bf16*)out, out_stride, (const bf16*)gate, gate_stride, H, window,
+                 sm_scale * kLog2e};
+#define LLB_WINDOW(DK, BN)                                                                                        \
+  if (dk == DK)                                                                                                   \
+    return dv == 64 ? launch<DK, 64, BN>(tq, tkv, p, B, max_q_len, st) : launch<DK, 128, BN>(tq, tkv, p, B, max_q_len, st);
+  LLB_WINDOW(64, 128)
+  LLB_WINDOW(128, 128)
+  LLB_WINDOW(192, 64)
+  LLB_WINDOW(256, 64)
+#undef LLB_WINDOW
+  return LLB_ERR_UNSUPPORTED;
 }

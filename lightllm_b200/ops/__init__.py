@@ -21,6 +21,7 @@ DTYPE_CODES = {torch.float32: 0, torch.bfloat16: 1}   # kernels that exist in bo
 
 import os as _os
 
+_ATTN_TC = _os.environ.get("LLB_ATTN_TC", "1") != "0"   # 0: prompt attention on the mma.sync kernel, for comparison
 _GEMM_DEBUG_TORCH = _os.environ.get("LLB_GEMM_DEBUG_TORCH", "0") == "1"
 
 # launch counter: the number of kernels of this package launched (claimed in bench output)
@@ -454,6 +455,14 @@ def gqa_prefill(q, kv_layer, req_to_token, b_req_idx, cu_q, b_ready_len, Hq, Hkv
     scale = sm_scale if sm_scale is not None else 1.0 / math.sqrt(D)
     if out is None:
         out = torch.empty((T, Hq, D), dtype=q.dtype, device=q.device)
+    if D == 128 and _ATTN_TC and scale > 0 and T > 0 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and \
+            out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and kv_layer.data_ptr() % 16 == 0:
+        check(kernels().llb_gqa_prefill_fa(ptr(q), i64(q.stride(0)), c_int(T), ptr(kv_layer), c_int(kv_layer.shape[0]),
+                                           ptr(req_to_token), i64(req_to_token.stride(0)), ptr(b_req_idx), ptr(cu_q),
+                                           ptr(b_ready_len), ptr(out), i64(out.stride(0)), c_int(B), c_int(max_q_len), c_int(Hq),
+                                           c_int(Hkv), f32(scale), stream()), "gqa_prefill_fa")
+        _count()
+        return out
     check(kernels().llb_gqa_prefill(ptr(q), i64(q.stride(0)), ptr(kv_layer), ptr(req_to_token),
                                     i64(req_to_token.stride(0)), ptr(b_req_idx), ptr(cu_q), ptr(b_ready_len),
                                     ptr(out), i64(out.stride(0)), c_int(B), c_int(max_q_len), c_int(Hq), c_int(Hkv),
