@@ -17,7 +17,7 @@ import math
 
 import torch
 
-from . import DTYPE_CODES, _count, gemm_f32
+from . import DTYPE_CODES, _count, gemm_f32, gemm_status
 from ._native import c_int, check, f32, i64, kernels, ptr, stream
 
 
@@ -47,6 +47,24 @@ def ref_mla_attention(q_lat, q_pe, kv_layer, req_to_token, b_req_idx, b_seq_len,
     return out
 
 
+MLA_DECODE_MIN_HEADS = 8   # not tried with fewer: the rest of the 128-row tile is empty
+
+
+def _mla_decode_rule(q_lat, q_pe, kv_layer, scale) -> bool:
+    """The tcgen05 decode kernel (`csrc/mla_decode.cu`): bf16, the heads of a token evenly spaced, TMA alignment."""
+    T, h, _ = q_lat.shape
+    return q_lat.dtype == torch.bfloat16 and h >= MLA_DECODE_MIN_HEADS and 0 < T <= 65535 and scale > 0 and \
+        kv_layer.is_contiguous() and q_pe.stride(0) == h * q_pe.stride(1) and q_pe.stride(1) % 8 == 0 and \
+        (q_lat.data_ptr() | q_pe.data_ptr() | kv_layer.data_ptr()) % 16 == 0
+
+
+def mla_decode_splits(T: int, h: int, max_kv_len: int) -> int:
+    """Shares of a request's keys: as many as fill 148 SMs with two CTAs (value halves) per request and 128 heads, at least two key
+    tiles each.  More would only add partial results, 128 KB per CTA."""
+    fill = 148 // (2 * T * -(-h // 128))
+    return max(1, min(fill, -(-max(max_kv_len, 1) // 128), 64))
+
+
 def mla_attention(q_lat, q_pe, kv_layer, req_to_token, b_req_idx, b_seq_len, cu_q, b_ready_len, kv_lora, scale,
                   is_prefill: bool, max_q_len: int = 1, max_kv_len: int = 0, batch_of=None):
     if not q_lat.is_cuda:
@@ -58,6 +76,18 @@ def mla_attention(q_lat, q_pe, kv_layer, req_to_token, b_req_idx, b_seq_len, cu_
     assert q_lat.is_contiguous() and q_pe.stride(-1) == 1
     out = torch.empty((T, h, kv_lora), dtype=q_lat.dtype, device=q_lat.device)
     B = b_req_idx.shape[0]
+    if not is_prefill and batch_of is None and _mla_decode_rule(q_lat, q_pe, kv_layer, scale):
+        splits = mla_decode_splits(T, h, max_kv_len)
+        po = pl = None
+        if splits > 1:
+            po = torch.empty(T * h * splits * kv_lora, dtype=torch.float32, device=q_lat.device)
+            pl = torch.empty(T * h * splits, dtype=torch.float32, device=q_lat.device)
+        check(kernels().llb_mla_decode(ptr(q_lat), ptr(q_pe), i64(q_pe.stride(0)), i64(q_pe.stride(1)), ptr(kv_layer),
+                                       c_int(kv_layer.shape[0]), ptr(req_to_token), i64(req_to_token.stride(0)), ptr(b_req_idx),
+                                       ptr(cu_q), ptr(b_ready_len), ptr(out), ptr(po), ptr(pl), c_int(T), c_int(h), c_int(splits),
+                                       f32(scale), ptr(gemm_status(q_lat.device)), stream()), "mla_decode")
+        _count(2 if splits > 1 else 1)
+        return out
     check(kernels().llb_mla_attention(ptr(q_lat), ptr(q_pe), i64(q_pe.stride(0)), i64(q_pe.stride(1)), ptr(kv_layer),
                                       ptr(req_to_token), i64(req_to_token.stride(0)), ptr(b_req_idx), ptr(cu_q),
                                       ptr(b_ready_len), ptr(batch_of), ptr(out), c_int(B), c_int(T), c_int(h),

@@ -1,0 +1,45 @@
+"""Decode attention of the latent cache on tcgen05 (csrc/mla_decode.cu) against fp32: head counts, tile edges, shares of the keys, a
+moving maximum."""
+import pytest
+import torch
+
+from lightllm_b200 import ops
+from lightllm_b200.ops import mla
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("lens", [[1], [63], [64, 65], [1, 128, 129, 1000, 2, 64], [3000, 5]])
+@pytest.mark.parametrize("h", [8, 16, 40, 128, 130])
+@pytest.mark.parametrize("splits,grow", [(0, False), (1, True), (5, True)])
+def test_matches_fp32(lens, h, splits, grow, monkeypatch):
+    B, nope = len(lens), 128
+    if splits:
+        monkeypatch.setattr(mla, "mla_decode_splits", lambda *a: splits)
+    g = torch.Generator(device="cuda").manual_seed(h)
+    n = sum(lens)
+    kv = torch.randn(n + 2, 1, 576, device="cuda", generator=g)
+    q_lat = torch.randn(B, h, 512, device="cuda", generator=g).to(BF)
+    q3 = torch.randn(B, h, nope + 64, device="cuda", generator=g).to(BF)
+    perm = torch.randperm(n, generator=torch.Generator().manual_seed(1)).to(torch.int32)
+    r2t = torch.zeros(B + 2, max(lens) + 3, dtype=torch.int32)
+    at = 0
+    for b, L in enumerate(lens):
+        r2t[b + 1, :L] = perm[at:at + L]
+        if grow:     # scores that grow along the context
+            kv[perm[at:at + L].long().cuda()] *= torch.linspace(0.05, 1.5, L, device="cuda").view(-1, 1, 1)
+        at += L
+    kv[n:] = float("nan")
+    kv = kv.to(BF)
+    rows = torch.arange(1, B + 1, dtype=torch.int32, device="cuda")
+    seq = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    cu = torch.arange(B + 1, dtype=torch.int32, device="cuda")
+    scale = 0.1 if grow else 192 ** -0.5
+    got = mla.mla_attention(q_lat, q3[:, :, nope:], kv, r2t.cuda(), rows, seq, cu, seq - 1, 512, scale, False, 1, max(lens)).float()
+    want = mla.ref_mla_attention(q_lat.float(), q3[:, :, nope:].float(), kv, r2t.cuda(), rows.cpu(), seq.cpu(), cu.cpu(), (seq - 1).cpu(),
+                                 512, scale)
+    # weights rounded to bf16 and one rounding of values of up to about 5
+    err = (got - want).abs().max().item()
+    assert err < 4e-2, (err, [(got - want)[i].abs().max().item() for i in range(B)])
+    assert int(ops.gemm_status("cuda:0").item()) == 0
