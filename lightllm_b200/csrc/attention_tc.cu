@@ -238,7 +238,7 @@ gqa_prefill_tc_kernel(const bf16* __restrict__ q, int64_t q_stride, const bf16* 
       if (lane == 0) mbar_arrive(v_full(stage));
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- MMA issuer: scores of tile s and P.V of tile t are issued in whichever order their inputs arrive ----
       constexpr uint32_t IDESC_S = umma_idesc(BM, BN, 1);
       constexpr uint32_t IDESC_PV = umma_idesc(BM, 64, 1) | (1u << 16);  // B operand MN-major

@@ -174,10 +174,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     }
     int stage = 0;
     uint32_t phase = 0;
+    const bool issuer = elect_one();
     for (int i = 0; i < nk; ++i) {
       const uint32_t sa = smem_base + stage * STAGE_BYTES;
       const int k = (kb0 + i) * BK;
-      if (lane == 0) {
+      if (issuer) {
         mbar_wait(empty_bar(stage), phase ^ 1, &abort_flag, p.status, 61);
         if (i >= STAGES || !ahead) {
           mbar_expect_tx(full_bar(stage), tx_bytes);
@@ -199,7 +200,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {  // ---- MMA issuer ----
+    if (elect_one()) {  // ---- MMA issuer ----
       int stage = 0;
       uint32_t phase = 0;
       for (int i = 0; i < nk; ++i) {

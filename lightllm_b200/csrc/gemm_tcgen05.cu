@@ -565,7 +565,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       int stage = 0;
@@ -610,7 +610,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -912,7 +912,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   if (warp == 0) {
     // ---- TMA producer (both CTAs) ----
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       int stage = 0;
@@ -936,7 +936,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       if (cta == 0) {
@@ -1156,7 +1156,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   const uint32_t tmem_base = tmem_base_slot;
 
   if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer (every CTA) ----
+    if (elect_one()) {  // ---- TMA producer (every CTA) ----
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       int stage = 0;
@@ -1184,7 +1184,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && half == 0) {  // ---- MMA issuer of the pair ----
+    if (half == 0 && elect_one()) {  // ---- MMA issuer of the pair ----
       int stage = 0;
       uint32_t phase = 0;
       for (int i = 0; i < nk; ++i) {
@@ -1522,7 +1522,7 @@ gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   const uint32_t tmem_base = tmem_base_slot;
 
   if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer ----
+    if (elect_one()) {  // ---- TMA producer ----
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       // The weights do not depend on the kernel before this one: the first stages' weight tiles are requested while
@@ -1558,7 +1558,7 @@ gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
   } else if (warp == 1) {
     pdl_wait();
-    if (lane == 0) {  // ---- MMA issuer ----
+    if (elect_one()) {  // ---- MMA issuer ----
       int stage = 0;
       uint32_t phase = 0;
       for (int i = 0; i < nk; ++i) {
@@ -1808,7 +1808,7 @@ gemm_bf16_pairsplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
   const uint32_t tmem_base = tmem_base_slot;
 
   if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer (both CTAs; transaction bytes are counted on the leader's barrier) ----
+    if (elect_one()) {  // ---- TMA producer (both CTAs; transaction bytes are counted on the leader's barrier) ----
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       const int wrow = n0 + (int)half * HALF;
@@ -1841,7 +1841,7 @@ gemm_bf16_pairsplit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
     }
   } else if (warp == 1) {
     pdl_wait();
-    if (lane == 0 && half == 0) {  // ---- MMA issuer of the pair ----
+    if (half == 0 && elect_one()) {  // ---- MMA issuer of the pair ----
       int stage = 0;
       uint32_t phase = 0;
       for (int i = 0; i < nk; ++i) {

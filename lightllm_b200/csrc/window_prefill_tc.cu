@@ -120,7 +120,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmKV);
       mbar_expect_tx(q_full, L::Q_BYTES);
@@ -145,7 +145,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- MMA issuer: scores of tile s and P.V of tile t are issued in whichever order their inputs arrive ----
       constexpr uint32_t IDESC_S = umma_idesc(BM, BN, 1);
       constexpr uint32_t IDESC_PV = umma_idesc(BM, 64, 1) | (1u << 16);  // B operand MN-major
