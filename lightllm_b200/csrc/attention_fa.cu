@@ -160,7 +160,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         const int ks = j % KS, vs = j % VS;
         const int r0 = next[0], r1 = next[1], r2 = next[2], r3 = next[3];
         if (j + 1 < n) fetch(j + 1);
-        mbar_wait(k_empty(ks), ((j / KS) & 1) ^ 1, abort_flag, status, 71);
+        if (!__all_sync(0xffffffffu, mbar_wait(k_empty(ks), ((j / KS) & 1) ^ 1, abort_flag, status, 71))) break;
         if (warp == 0 && lane == 0) mbar_expect_tx(k_full(ks), L::K_BYTES);
         if (active)
 #pragma unroll
@@ -168,7 +168,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             tma_gather4(smem_base + L::OFF_K + ks * L::K_BYTES + c * BN * 128 + quad * 512, &tmKV, k_full(ks), k_col + c * 64, r0, r1,
                         r2, r3);
         __syncwarp();
-        mbar_wait(v_empty(vs), ((j / VS) & 1) ^ 1, abort_flag, status, 72);
+        if (!__all_sync(0xffffffffu, mbar_wait(v_empty(vs), ((j / VS) & 1) ^ 1, abort_flag, status, 72))) break;
         if (warp == 0 && lane == 0) mbar_expect_tx(v_full(vs), L::V_BYTES);
         if (active)
 #pragma unroll
@@ -181,7 +181,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int row0 = p.cu_kv[b];
       for (int j = 0; j < n; ++j) {
         const int ks = j % KS, vs = j % VS;
-        mbar_wait(k_empty(ks), ((j / KS) & 1) ^ 1, abort_flag, status, 71);
+        if (!mbar_wait(k_empty(ks), ((j / KS) & 1) ^ 1, abort_flag, status, 71)) break;
         mbar_expect_tx(k_full(ks), L::K_BYTES);
 #pragma unroll
         for (int c = 0; c < DK / 64; ++c) {
@@ -189,7 +189,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tma_load_2d(smem_base + L::OFF_K + ks * L::K_BYTES + c * BN * 128, mine ? &tmKV : &tmShared, k_full(ks),
                       mine ? y * p.own + c * 64 : p.shared_col + c * 64 - p.own, row0 + j * BN);
         }
-        mbar_wait(v_empty(vs), ((j / VS) & 1) ^ 1, abort_flag, status, 72);
+        if (!mbar_wait(v_empty(vs), ((j / VS) & 1) ^ 1, abort_flag, status, 72)) break;
         mbar_expect_tx(v_full(vs), L::V_BYTES);
 #pragma unroll
         for (int c = 0; c < DV / 64; ++c)
@@ -234,7 +234,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       scores(0, 0);
       if (n1 > 0) scores(1, 0);
       umma_commit(k_empty(0));
-      for (int j = 0; j < n; ++j) {
+      for (int j = 0; j < n && !*abort_flag; ++j) {
         const bool k_next = j + 1 < n;
         if (j < n0) {
           values(0, j);
@@ -356,6 +356,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag) settle_after_abort();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);

@@ -178,8 +178,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     for (int i = 0; i < nk; ++i) {
       const uint32_t sa = smem_base + stage * STAGE_BYTES;
       const int k = (kb0 + i) * BK;
+      const bool free = !issuer || mbar_wait(empty_bar(stage), phase ^ 1, &abort_flag, p.status, 61);
+      if (MODE == GATHER ? !__all_sync(0xffffffffu, free) : !free) break;
       if (issuer) {
-        mbar_wait(empty_bar(stage), phase ^ 1, &abort_flag, p.status, 61);
         if (i >= STAGES || !ahead) {
           mbar_expect_tx(full_bar(stage), tx_bytes);
           tma_load_2d(sa, &tmW, full_bar(stage), k, w_row0);
@@ -189,7 +190,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           for (int g = 0; g < groups16; ++g) tma_load_2d(sa + W_BYTES + g * 16 * ROW, &tmX, full_bar(stage), k, row0 + g * 16);
       }
       if (MODE == GATHER) {
-        __syncwarp();
+        __syncwarp();  // the expected bytes before the copies
         if (lane < groups16 * 4)
           tma_gather4(sa + W_BYTES + lane * 4 * ROW, &tmX, full_bar(stage), k, r4[0], r4[1], r4[2], r4[3]);
       }
@@ -365,6 +366,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       }
     }
   }
+  if (*(volatile int*)&abort_flag) settle_after_abort();
   cluster_sync_all();  // nobody leaves while a peer may still read its share
   if (warp == 1) {
     tc_fence_after();

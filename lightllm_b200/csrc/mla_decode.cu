@@ -60,8 +60,10 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   auto full = [&](int s) { return bar + 8 * s; };
   auto empty = [&](int s) { return bar + 8 * (2 + s); };
   auto s_full = [&](int s) { return bar + 8 * (4 + s); };
-  const uint32_t p_full = bar + 8 * 6, o_full = bar + 8 * 7, q_full = bar + 8 * 8, qt_full = bar + 8 * 9,
-                 done = bar + 8 * 10;
+  // one per score buffer: the scores of a tile may be there before all warps have finished with the tile before it, and a warp that runs
+  // ahead (another one may be rescaling) must not be counted for it
+  auto p_full = [&](int s) { return bar + 8 * (6 + s); };
+  const uint32_t o_full = bar + 8 * 8, q_full = bar + 8 * 9, qt_full = bar + 8 * 10, done = bar + 8 * 11;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_BAR + 128);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 132);
 
@@ -70,8 +72,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int s = 0; s < 2; ++s) mbar_init(full(s), 1), mbar_init(empty(s), 1), mbar_init(s_full(s), 1);
-    mbar_init(p_full, 4);
+    for (int s = 0; s < 2; ++s) mbar_init(full(s), 1), mbar_init(empty(s), 1), mbar_init(s_full(s), 1), mbar_init(p_full(s), 4);
     mbar_init(o_full, 1);
     mbar_init(done, 1);
     mbar_init(q_full, 1);
@@ -126,7 +127,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int s = j & 1;
       const int r0 = next[0], r1 = next[1], r2 = next[2], r3 = next[3];
       if (j + 1 < n) fetch(j + 1);
-      mbar_wait(empty(s), ((j >> 1) & 1) ^ 1, abort_flag, p.status, 81);
+      if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ((j >> 1) & 1) ^ 1, abort_flag, p.status, 81))) break;
       if (w == 0 && lane == 0) mbar_expect_tx(full(s), STAGE);
       if (active) tma_gather4(smem_base + OFF_K + s * STAGE + c * BLOCK + quad * 512, &tmKV, full(s), c * 64, r0, r1, r2, r3);
       __syncwarp();
@@ -158,7 +159,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       scores(0);
       for (int j = 0; j < n; ++j) {
         if (j + 1 < n) scores(j + 1);
-        mbar_wait(p_full, j & 1, abort_flag, p.status, 85);
+        if (!mbar_wait(p_full(j & 1), (j >> 1) & 1, abort_flag, p.status, 85)) break;
         tc_fence_after();
         const uint32_t v = smem_base + OFF_K + (j & 1) * STAGE + half * 4 * BLOCK;
         const uint64_t dv = umma_smem_desc_sw128_mn(v);
@@ -198,7 +199,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     float m = -INFINITY, l = 0.f;
     for (int j = 0; j < n; ++j) {
       const uint32_t t_s = t_lane + S_COL + (j & 1) * BN;
-      mbar_wait(s_full(j & 1), (j >> 1) & 1, abort_flag, p.status, 86);
+      if (!__all_sync(0xffffffffu, mbar_wait(s_full(j & 1), (j >> 1) & 1, abort_flag, p.status, 86))) break;
       tc_fence_after();
       uint32_t s[BN];
       tmem_ld_32x32(t_s, s);
@@ -252,7 +253,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(p_full(j & 1));
     }
     // not o_full: the scores of the last tile were issued ahead of the last but one P . V, so o_full may be two phases behind here
     mbar_wait(done, 0, abort_flag, p.status, 88);
@@ -291,6 +292,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag) settle_after_abort();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);

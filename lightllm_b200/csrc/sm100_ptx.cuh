@@ -86,6 +86,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// After a wait that ran out, once the CTA's warps issue nothing more: a millisecond for the copies and MMAs in flight to end before
+// their shared and tensor memory is given back.
+__device__ __forceinline__ void settle_after_abort() {
+  const uint64_t t0 = global_timer_ns();
+  while (global_timer_ns() - t0 < 1000000ull) {
+  }
+}
+
 // 2-D TMA tile load, completion counted on an mbarrier of this CTA. x = innermost coordinate.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(

@@ -43,3 +43,31 @@ def test_matches_fp32(lens, h, splits, grow, monkeypatch):
     err = (got - want).abs().max().item()
     assert err < 4e-2, (err, [(got - want)[i].abs().max().item() for i in range(B)])
     assert int(ops.gemm_status("cuda:0").item()) == 0
+
+
+@pytest.mark.parametrize("B", [1, 96])
+@pytest.mark.parametrize("first", [0, 32, 64, 96])
+def test_one_warp_rescales(B, first):
+    """The maximum of 32 heads (a warp's rows) moves in every tile, that of the others never: a warp that is a tile ahead must not be
+    counted for the one that lags."""
+    L, h, nope, a = 3000, 128, 128, 6.8    # scores grow by 590 (as powers of two) over 47 tiles: 12.6 a tile, the threshold is 8
+    g = torch.Generator(device="cuda").manual_seed(first)
+    sign = torch.randint(0, 2, (576,), device="cuda", generator=g).float() * 2 - 1
+    kv = torch.linspace(0.05, 1.5, L, device="cuda")[:, None] * sign + 0.1 * torch.randn(L, 576, device="cuda", generator=g)
+    kv = kv.view(L, 1, 576).to(BF)
+    q = 0.05 * torch.randn(B, h, 576, device="cuda", generator=g)
+    q[:, first:first + 32] = a * sign
+    q_lat = q[:, :, :512].to(BF).contiguous()
+    q3 = torch.zeros(B, h, nope + 64, device="cuda", dtype=BF)
+    q3[:, :, nope:] = q[:, :, 512:].to(BF)
+    r2t = torch.arange(L, dtype=torch.int32, device="cuda").expand(B, L).contiguous()
+    rows = torch.arange(B, dtype=torch.int32, device="cuda")
+    seq = torch.full((B,), L, dtype=torch.int32, device="cuda")
+    cu = torch.arange(B + 1, dtype=torch.int32, device="cuda")
+    f = lambda: mla.mla_attention(q_lat, q3[:, :, nope:], kv, r2t, rows, seq, cu, seq - 1, 512, 192 ** -0.5, False, 1, L)  # noqa: E731
+    outs = [f() for _ in range(4)]
+    s = torch.einsum("bhd,ld->bhl", torch.cat([q_lat, q3[:, :, nope:]], 2).double(), kv[:, 0].double()) * 192 ** -0.5
+    want = torch.einsum("bhl,ld->bhd", torch.softmax(s, -1), kv[:, 0, :512].double())
+    assert (outs[0].double() - want).abs().max().item() < 2e-2   # weights and outputs (up to 1.8) rounded to bf16
+    assert all(torch.equal(outs[0], o) for o in outs)
+    assert int(ops.gemm_status("cuda:0").item()) == 0
