@@ -1,6 +1,6 @@
 // Prefill attention on the 5th-generation tensor cores (tcgen05 + tensor memory), causal, varlen, aware of an already cached
-// prefix, K/V read through the token-granular slot table of the KV pool: the windowed form (plain attention of head size 128 is
-// attention_fa.cu) with key sizes up to 256, any multiple of 64 as value size, chunks of positions, kept first positions, biases by distance, soft-capped scores, and
+// prefix, K/V read through the token-granular slot table of the KV pool.  Head size 128, and a windowed form with key sizes
+// up to 256, any multiple of 64 as value size, chunks of positions, kept first positions, biases by distance, soft-capped scores, and
 // a sigmoid gate on the output.
 //
 // One CTA computes 128 query rows of one (request, query head).  Per 128-key tile (64 keys for key sizes above 128):
@@ -495,6 +495,19 @@ LLB_EXPORT int llb_attn_tc_status() {
   int v = 0;
   cudaMemcpyFromSymbol(&v, g_attn_tc_status, sizeof(int));
   return v;
+}
+
+// Same contract as llb_gqa_prefill (head size 128 only): q [T, Hq, 128] new tokens of all requests back to back.
+LLB_EXPORT int llb_gqa_prefill_tc(const void* q, int64_t q_stride, const void* kv_layer, const int* req_to_token,
+                                  int64_t r2t_stride, const int* b_req_idx, const int* cu_q, const int* b_ready_len,
+                                  void* out, int64_t out_stride, int B, int max_q_len, int Hq, int Hkv, float sm_scale,
+                                  cudaStream_t st) {
+  if (B <= 0 || max_q_len <= 0) return LLB_OK;
+  if (!(sm_scale > 0.f) || Hkv <= 0 || Hq % Hkv != 0 || (q_stride % 8) || (out_stride % 8) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15))
+    return LLB_ERR_BAD_ARG;
+  return launch_tc<128, 128, 128, false, false>((const bf16*)q, q_stride, (const bf16*)kv_layer, req_to_token, r2t_stride, b_req_idx,
+                                         cu_q, b_ready_len, (bf16*)out, out_stride, B, max_q_len, Hq, Hkv, sm_scale, 1, KeyRule{},
+                                         OutGate{nullptr, 0, 1.f, 0}, st);
 }
 
 // Key size dk (64, 128, 192, 256), value size dv (a multiple of 64), window or chunk (0: none), first `keep` positions always seen,
