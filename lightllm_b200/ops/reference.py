@@ -284,7 +284,7 @@ def sample(logits, temperature=None, top_p=None, top_k=None, seeds=None, steps=N
 def greedy_partials(logits, idx_off, splits):
     """[B, S, 3]: (max, arg-max global id as float bits, sum exp(x - max)) of S column slices."""
     B, V = logits.shape
-    per = ((V + splits - 1) // splits + 3) & ~3
+    per = ((V + splits - 1) // splits + 7) & ~7
     out = torch.zeros((B, splits, 3), dtype=torch.float32, device=logits.device)
     for s in range(splits):
         i0, i1 = s * per, min(V, (s + 1) * per)

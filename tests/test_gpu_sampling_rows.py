@@ -55,3 +55,21 @@ def test_draws(V, dtype):
         assert key[i] > best - 1e-3                      # the winner (or one within rounding of it) ...
         edge = x.cpu().numpy()[keep].min()
         assert float(x[i]) > edge - 1e-4                 # ... of the kept tokens
+
+
+@pytest.mark.parametrize("V,pad", [(1, 0), (7, 0), (2049, 0), (4099, 5), (40000, 0), (128256, 8), (128257, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_greedy(V, pad, dtype):
+    """The arg-max (the first of equal ones) and its log-probability, rows on any boundary, logits of -inf among them."""
+    B = 5
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = (torch.randn(B, V + pad, device="cuda", generator=g) * 4).to(dtype)[:, :V]
+    x[1] = 0                       # all equal
+    x[2, : V // 2] = float("-inf")
+    x[3, V - 1] = 50
+    x[4, : V - 1] = float("-inf")
+    ids, lp = ops.sample(x)
+    want = torch.stack([(r == r.max()).nonzero()[0, 0] for r in x])
+    assert torch.equal(ids, want)
+    ref_lp = torch.log_softmax(x.double(), -1).gather(1, want[:, None])[:, 0]
+    assert (lp.double() - ref_lp).abs().max().item() < 1e-4   # fp32 sums of up to 1e5 positive terms, fast exp and log
