@@ -235,8 +235,32 @@ mla_rope_kv_scatter_kernel(bf16* __restrict__ q3, int64_t q_st, int64_t q_sh, co
   const int half = rope >> 1;
   const float* cr = cos_t + (int64_t)pos[t] * half;
   const float* sr = sin_t + (int64_t)pos[t] * half;
-  // q: pairs (i, i + half) of every head
-  for (int idx = threadIdx.x; idx < hq * half; idx += blockDim.x) {
+  // q: pairs (i, i + half) of every head, eight at a time where the heads' rotated parts and the tables start on 16-byte boundaries
+  // (one by one, 16 rounds of dependent 2-byte accesses a token, took 90 us for 5000 tokens of 128 heads)
+  const bool vec = (half & 7) == 0 && (nope & 7) == 0 && (q_st & 7) == 0 && (q_sh & 7) == 0 &&
+                   (((uintptr_t)q3 | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0;
+  const int octets = half >> 3;
+  for (int idx = threadIdx.x; vec && idx < hq * octets; idx += blockDim.x) {
+    const int h = idx / octets, i = (idx - h * octets) * 8;
+    bf16* p = q3 + (int64_t)t * q_st + (int64_t)h * q_sh + nope + i;
+    float x1[8], x2[8];
+    unpack8(*reinterpret_cast<const bf16x8*>(p), x1);
+    unpack8(*reinterpret_cast<const bf16x8*>(p + half), x2);
+#pragma unroll
+    for (int k = 0; k < 8; k += 4) {
+      const float4 c4 = *reinterpret_cast<const float4*>(cr + i + k), s4 = *reinterpret_cast<const float4*>(sr + i + k);
+      const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float a = x1[k + e], b = x2[k + e];
+        x1[k + e] = a * c[e] - b * s[e];
+        x2[k + e] = b * c[e] + a * s[e];
+      }
+    }
+    *reinterpret_cast<bf16x8*>(p) = pack8(x1);
+    *reinterpret_cast<bf16x8*>(p + half) = pack8(x2);
+  }
+  for (int idx = threadIdx.x; !vec && idx < hq * half; idx += blockDim.x) {
     int h = idx / half, i = idx % half;
     bf16* p = q3 + (int64_t)t * q_st + (int64_t)h * q_sh + nope;
     float x1 = __bfloat162float(p[i]), x2 = __bfloat162float(p[i + half]);

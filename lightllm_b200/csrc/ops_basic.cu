@@ -172,15 +172,30 @@ __global__ void __launch_bounds__(256) rope_kv_scatter_kernel(bf16* __restrict__
   bf16* row = qkv + (int64_t)t * qkv_stride;
   const float* cr = cos_t + (int64_t)p * half;
   const float* sr = sin_t + (int64_t)p * half;
+  const bool table16 = (((uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0;  // rows are multiples of 32 bytes
+  // a thread's vectors of AHEAD rounds are fetched before the first of them is worked on: a token has only a few rounds, and one after
+  // the other they cost a memory latency each
+  constexpr int AHEAD = 4;
   const int iters = cdiv(total, (int)blockDim.x);
+  bf16x8 raws[AHEAD];
   for (int it = 0; it < iters; ++it) {
     int item = threadIdx.x + it * blockDim.x;
+    if (it % AHEAD == 0) {
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const int i = item + u * (int)blockDim.x;
+        if (it + u < iters) raws[u] = reinterpret_cast<const bf16x8*>(row)[i < total ? i : item % LANES_PER_HEAD];
+      }
+    }
     bool valid = item < total;
     int head = valid ? item / LANES_PER_HEAD : 0;
     int v = item % LANES_PER_HEAD;
     int kind = head < Hq ? 0 : (head < Hq + Hkv ? 1 : 2);  // q, k, v
     float x[8];
-    bf16x8 raw = reinterpret_cast<const bf16x8*>(row + (int64_t)head * D)[v];
+    bf16x8 raw = raws[0];
+#pragma unroll
+    for (int u = 1; u < AHEAD; ++u)
+      if (it % AHEAD == u) raw = raws[u];
     unpack8(raw, x);
     const bf16* nw = kind == 0 ? q_norm_w : (kind == 1 ? k_norm_w : nullptr);
     // the whole warp runs the shuffles (heads of different kinds share a warp)
@@ -210,11 +225,20 @@ __global__ void __launch_bounds__(256) rope_kv_scatter_kernel(bf16* __restrict__
     for (int k = 0; k < 8; ++k) y[k] = __shfl_sync(0xffffffffu, x[k], partner & 31);
     if (rotary) {
       int base = (lower ? v : v - half_lanes) * 8;
+      float cs[8], sn[8];
+      if (table16) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        float c = cr[base + k], sn = sr[base + k];
-        x[k] = lower ? (x[k] * c - y[k] * sn) : (x[k] * c + y[k] * sn);
+        for (int k = 0; k < 8; k += 4) {
+          const float4 c4 = *reinterpret_cast<const float4*>(cr + base + k), s4 = *reinterpret_cast<const float4*>(sr + base + k);
+          cs[k] = c4.x, cs[k + 1] = c4.y, cs[k + 2] = c4.z, cs[k + 3] = c4.w;
+          sn[k] = s4.x, sn[k + 1] = s4.y, sn[k + 2] = s4.z, sn[k + 3] = s4.w;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) cs[k] = cr[base + k], sn[k] = sr[base + k];
       }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = lower ? (x[k] * cs[k] - y[k] * sn[k]) : (x[k] * cs[k] + y[k] * sn[k]);
     }
     bf16x8 o = pack8(x);
     float amax = 0.f;
