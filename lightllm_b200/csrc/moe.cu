@@ -298,19 +298,122 @@ moe_table_align_kernel(const TableRoute* __restrict__ routes, const int64_t* __r
       n, r.e0, r.E_local, m_pad, sorted_pair, pair_row, mblock, off, off + r.E_local + 1);
 }
 
-// A_sorted[row] = x[sorted_pair[row] / k]  (zeros for padding rows)
+// The same layout from a cluster of 8 CTAs for the many pairs of a prompt pass (one CTA took 60 us for 65536): every CTA counts its
+// part of the pairs, the counts are read through distributed shared memory, and a CTA's rows of an expert follow those of the CTAs
+// before it.
+constexpr int kAlignCtas = 8;
+__device__ __forceinline__ int peer_int(const int* local, int rank) {
+  uint32_t a;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void align_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__global__ void __cluster_dims__(kAlignCtas, 1, 1) __launch_bounds__(1024)
+moe_align_cluster_kernel(const int* __restrict__ ids, int n_pairs, int e0, int E_local, int m_pad,
+                         int* __restrict__ sorted_pair, int* __restrict__ pair_row, int* __restrict__ mblock_expert,
+                         int* __restrict__ expert_off, int* __restrict__ total_rows) {
+  extern __shared__ int sm[];
+  int* cnt = sm;                    // [E_local] my pairs
+  int* off = sm + E_local;          // [E_local + 1] first row of an expert
+  int* cur = sm + 2 * E_local + 1;  // [E_local] next row of mine
+  const int rank = blockIdx.x;
+  const int each = (n_pairs + kAlignCtas - 1) / kAlignCtas, p0 = min(n_pairs, rank * each), p1 = min(n_pairs, p0 + each);
+  auto expert = [&](int p) {
+    const int e = ids[p] < 0 ? -1 : LLB_CHECK_EXPERT(ids[p]) - e0;
+    return e >= 0 && e < E_local ? e : -1;
+  };
+  for (int i = threadIdx.x; i < E_local; i += blockDim.x) cnt[i] = 0;
+  for (int r = rank * blockDim.x + threadIdx.x; r < m_pad; r += kAlignCtas * blockDim.x) sorted_pair[r] = -1;
+  __syncthreads();
+  for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
+    const int e = expert(p);
+    if (e >= 0) atomicAdd(&cnt[e], 1);
+  }
+  align_barrier();  // the counts of all CTAs are there, and sorted_pair is cleared
+  for (int e = threadIdx.x; e < E_local; e += blockDim.x) {
+    int before = 0, all = 0;
+    for (int r = 0; r < kAlignCtas; ++r) {
+      const int c = peer_int(cnt + e, r);
+      if (r < rank) before += c;
+      all += c;
+    }
+    cur[e] = before;
+    off[e] = (all + 127) / 128 * 128;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {  // exclusive prefix sum over the experts
+    int acc = 0;
+    for (int e = threadIdx.x; e < (E_local + 31) / 32 * 32; e += 32) {
+      const int v = e < E_local ? off[e] : 0;
+      int upto = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, upto, o);
+        if ((int)threadIdx.x >= o) upto += u;
+      }
+      if (e < E_local) off[e] = acc + upto - v;
+      acc += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (threadIdx.x == 0) off[E_local] = acc;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E_local; e += blockDim.x) cur[e] += off[e];
+  if (rank == 0) {
+    for (int i = threadIdx.x; i <= E_local; i += blockDim.x) expert_off[i] = off[i];
+    if (threadIdx.x == 0) total_rows[0] = off[E_local];
+  }
+  for (int b = rank * blockDim.x + threadIdx.x; b < m_pad / 128; b += kAlignCtas * blockDim.x) {
+    const int row = b * 128;
+    int e = -1;
+    if (row < off[E_local]) {  // the last expert that starts at or before the row
+      int lo = 0, hi = E_local - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (off[mid] <= row) lo = mid; else hi = mid - 1;
+      }
+      e = lo;
+    }
+    mblock_expert[b] = e;
+  }
+  __syncthreads();
+  for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
+    const int e = expert(p);
+    int r = -1;
+    if (e >= 0) {
+      r = atomicAdd(&cur[e], 1);
+      sorted_pair[r] = p;
+    }
+    pair_row[p] = r;
+  }
+  align_barrier();  // nobody leaves while a peer may still read its counts
+}
+
+// A_sorted[row] = x[sorted_pair[row] / k]; padding rows are zeroed, or left as they are (zero_pad 0).  A warp per row, eight 16-byte
+// loads in flight per lane.
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(bf16* __restrict__ a_sorted, const bf16* __restrict__ x, const int* __restrict__ sorted_pair,
-                  const int* __restrict__ total_rows, int k, int H_vec, int64_t x_stride_vec) {
-  const int rows = total_rows[0];
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+                  const int* __restrict__ total_rows, int k, int H_vec, int64_t x_stride_vec, int zero_pad) {
+  const int rows = total_rows[0], lane = threadIdx.x & 31;
+  constexpr int U = 8;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {
     const int p = sorted_pair[r];
+    if (p < 0 && !zero_pad) continue;
     uint4* dst = reinterpret_cast<uint4*>(a_sorted) + (int64_t)r * H_vec;
-    if (p < 0) {
-      for (int v = threadIdx.x; v < H_vec; v += blockDim.x) dst[v] = make_uint4(0, 0, 0, 0);
-    } else {
-      const uint4* src = reinterpret_cast<const uint4*>(x) + (int64_t)(p / k) * x_stride_vec;
-      for (int v = threadIdx.x; v < H_vec; v += blockDim.x) dst[v] = src[v];
+    const uint4* src = reinterpret_cast<const uint4*>(x) + (int64_t)(p < 0 ? 0 : p / k) * x_stride_vec;
+    for (int v0 = lane; v0 < H_vec; v0 += 32 * U) {
+      uint4 w[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        w[u] = make_uint4(0, 0, 0, 0);
+        if (p >= 0 && v0 + 32 * u < H_vec) w[u] = src[v0 + 32 * u];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v0 + 32 * u < H_vec) dst[v0 + 32 * u] = w[u];
     }
   }
 }
@@ -435,21 +538,29 @@ LLB_EXPORT int llb_moe_align(const int* ids, int n_pairs, int e0, int E_local, i
                              int* pair_row, int* mblock_expert, int* expert_off, int* total_rows, cudaStream_t st) {
   if (E_local > 2048 || m_pad % 128 != 0) return LLB_ERR_UNSUPPORTED;
   int smem = (3 * E_local + 1) * sizeof(int);
-  moe_align_kernel<<<1, 1024, smem, st>>>(ids, n_pairs, e0, E_local, m_pad, sorted_pair, pair_row, mblock_expert,
-                                          expert_off, total_rows);
+  if (n_pairs >= 4096)
+    moe_align_cluster_kernel<<<kAlignCtas, 1024, smem, st>>>(ids, n_pairs, e0, E_local, m_pad, sorted_pair, pair_row, mblock_expert,
+                                                             expert_off, total_rows);
+  else
+    moe_align_kernel<<<1, 1024, smem, st>>>(ids, n_pairs, e0, E_local, m_pad, sorted_pair, pair_row, mblock_expert,
+                                            expert_off, total_rows);
   LLB_LAUNCH_CHECK();
   return LLB_OK;
 }
 
-LLB_EXPORT int llb_moe_gather(void* a_sorted, const void* x, const int* sorted_pair, const int* total_rows, int k,
-                              int H, int64_t x_stride, int max_rows, cudaStream_t st) {
+LLB_EXPORT int llb_moe_gather_rows(void* a_sorted, const void* x, const int* sorted_pair, const int* total_rows, int k,
+                                   int H, int64_t x_stride, int max_rows, int zero_pad, cudaStream_t st) {
   if (max_rows <= 0) return LLB_OK;
   if (H % 8 || x_stride % 8) return LLB_ERR_UNSUPPORTED;
-  int blocks = max_rows < 148 * 8 ? max_rows : 148 * 8;
+  const int blocks = cdiv(max_rows, 8) < 148 * 8 ? cdiv(max_rows, 8) : 148 * 8;
   moe_gather_kernel<<<blocks, 256, 0, st>>>((bf16*)a_sorted, (const bf16*)x, sorted_pair, total_rows, k, H / 8,
-                                            x_stride / 8);
+                                            x_stride / 8, zero_pad);
   LLB_LAUNCH_CHECK();
   return LLB_OK;
+}
+LLB_EXPORT int llb_moe_gather(void* a_sorted, const void* x, const int* sorted_pair, const int* total_rows, int k,
+                              int H, int64_t x_stride, int max_rows, cudaStream_t st) {
+  return llb_moe_gather_rows(a_sorted, x, sorted_pair, total_rows, k, H, x_stride, max_rows, 1, st);
 }
 
 LLB_EXPORT int llb_moe_combine(void* out, const void* y, const int* pair_row, const float* weights, int T, int k, int H,

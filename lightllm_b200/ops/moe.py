@@ -175,14 +175,14 @@ def gemm_grouped(a_sorted, w_stacked, mblock_expert, n_per_expert: int, epi: str
     return out
 
 
-def gather_rows(x, lay: MoeLayout):
-    """The rows of x in expert-sorted order (zero rows for padding)."""
+def gather_rows(x, lay: MoeLayout, zero_pad: bool = True):
+    """The rows of x in expert-sorted order (zero rows for padding; zero_pad False: padding rows undefined)."""
     T, H = x.shape
     a = torch.empty((lay.m_pad, H), dtype=x.dtype, device=x.device)
     halves = x.element_size() // 2          # the kernel counts 2-byte elements
-    check(kernels().llb_moe_gather(ptr(a), ptr(x), ptr(lay.sorted_pair), ptr(lay.total_rows), c_int(lay.k),
-                                   c_int(H * halves), i64(x.stride(0) * halves), c_int(lay.m_pad), stream()),
-          "moe_gather")
+    check(kernels().llb_moe_gather_rows(ptr(a), ptr(x), ptr(lay.sorted_pair), ptr(lay.total_rows), c_int(lay.k),
+                                        c_int(H * halves), i64(x.stride(0) * halves), c_int(lay.m_pad), c_int(int(zero_pad)),
+                                        stream()), "moe_gather")
     _count()
     return a
 
@@ -244,15 +244,15 @@ def fused_experts(x, w13, w2, ids, weights, act="silu", e0: int = 0, out=None, a
     E_local, N13, _ = w13.shape
     I = N13 // 2
     k = ids.shape[1]
-    lay = moe_align(ids, E_local, e0)
     few = T <= FEW_TOKENS and x.dtype == torch.bfloat16 and x.stride(1) == 1 and b13 is None and b2 is None and \
         (act == "silu" or act == "gelu" and not fp8_w) and N13 % 64 == 0 and H % 16 == 0 and I % 16 == 0 and \
         (x.stride(0) * 2) % 16 == 0 and x.data_ptr() % 16 == 0
+    lay = moe_align(ids, E_local, e0)
     if few:
         y = _few_tokens_experts(x, w13, w2, lay, act)
         a = None
     else:
-        a = gather_rows(x, lay)
+        a = gather_rows(x, lay, zero_pad=False)   # rows do not mix until the combination, which reads the valid ones
     if few:
         pass
     elif fp8_w:
