@@ -456,10 +456,12 @@ constexpr int kRegSmemBytes = 4 * kRegWarpBytes;
 template <bool FP8>
 __device__ __forceinline__ void cvt_k_word(uint32_t w, uint32_t& b0, uint32_t& b1) {
   if (FP8) {
-    __half2_raw a = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w & 0xffffu), __NV_E4M3);
-    __half2_raw b = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> 16), __NV_E4M3);
-    b0 = (uint32_t)a.x | ((uint32_t)a.y << 16);
-    b1 = (uint32_t)b.x | ((uint32_t)b.y << 16);
+    asm("{\n\t.reg .b16 lo, hi;\n\t"
+        "mov.b32 {lo, hi}, %2;\n\t"
+        "cvt.rn.f16x2.e4m3x2 %0, lo;\n\t"
+        "cvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
+        : "=r"(b0), "=r"(b1)
+        : "r"(w));
   } else {
     const __half2 bias = __halves2half2(__ushort_as_half((unsigned short)0x6480), __ushort_as_half((unsigned short)0x6480));
     const uint32_t x = w ^ 0x80808080u;
@@ -477,8 +479,13 @@ template <bool FP8>
 __device__ __forceinline__ uint32_t cvt_v_pair(uint32_t a, uint32_t b, int i) {
   const uint32_t p = __byte_perm(a, b, (uint32_t)(i | ((4 + i) << 4)));   // low 16 bits: {a.byte i, b.byte i}
   if (FP8) {
-    __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(p & 0xffffu), __NV_E4M3);
-    return (uint32_t)h.x | ((uint32_t)h.y << 16);
+    uint32_t h;
+    asm("{\n\t.reg .b16 lo, hi;\n\t"
+        "mov.b32 {lo, hi}, %1;\n\t"
+        "cvt.rn.f16x2.e4m3x2 %0, lo;\n\t}"
+        : "=r"(h)
+        : "r"(p));
+    return h;
   } else {
     const __half2 bias = __halves2half2(__ushort_as_half((unsigned short)0x6480), __ushort_as_half((unsigned short)0x6480));
     uint32_t q = __byte_perm(p ^ 0x00008080u, 0x64646464u, 0x4140);
@@ -688,12 +695,14 @@ gqa_decode_q8_regs_kernel(const bf16* __restrict__ q, int64_t q_stride, const in
       }
       l_run[r] = l_run[r] * alpha[r] + rs;
     }
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {  // the maxima settle after a few tiles
 #pragma unroll
-    for (int nt = 0; nt < 16; ++nt) {
-      o[nt][0] *= alpha[0];
-      o[nt][1] *= alpha[0];
-      o[nt][2] *= alpha[1];
-      o[nt][3] *= alpha[1];
+      for (int nt = 0; nt < 16; ++nt) {
+        o[nt][0] *= alpha[0];
+        o[nt][1] *= alpha[0];
+        o[nt][2] *= alpha[1];
+        o[nt][3] *= alpha[1];
+      }
     }
     const uint32_t a0 = pack_f16x2(s[0][0] * vs[0][0], s[0][1] * vs[0][1]);
     const uint32_t a1 = pack_f16x2(s[0][2] * vs[0][0], s[0][3] * vs[0][1]);
