@@ -2078,6 +2078,8 @@ LLB_EXPORT int llb_gemm_set_push(void** push, void** cnt, int rank, int world, i
   g_push.max_mb = max_mb;
   return LLB_OK;
 }
+// Ranks of the push that the next GEMM has to make (0: none); only the kernels of this file make it.
+LLB_EXPORT int llb_gemm_push_armed() { return g_push.world; }
 
 // C[M,N] (ldc) = A[M,K] (lda) . W[N,K]^T (ldw)  with epilogue `epi`:
 //   0 store bf16 (+bias)          1 store bf16 of acc (+bias) + residual[M,N] (same ldc)

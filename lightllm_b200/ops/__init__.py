@@ -281,7 +281,8 @@ def gemm(a, w, epi: str = "store", residual=None, bias=None, out=None, bn: int =
         return res
     M, K = a.shape
     N = w.shape[0]
-    if stream_k == 0 and not isinstance(w, TiledWeight) and (4000 <= bn < 4100 or bn == 0 and _stream_rule(M, N, K, epi, bias)):
+    if stream_k == 0 and not isinstance(w, TiledWeight) and (4000 <= bn < 4100 or bn == 0 and _stream_rule(M, N, K, epi, bias)) and \
+            not kernels().llb_gemm_push_armed():   # a push set up for this call: the tile kernels make it
         if bn == 0:   # a stored variant of this kernel is a number of K shares; other variants were tuned before it was there
             bn = _tuned_bn(M, N, K, epi) if bias is None else 0
         return _gemm_stream(a, w, epi, residual, bias, out, bn - 4000 if 4000 <= bn < 4100 else 0, w_ready)

@@ -123,7 +123,7 @@ class FusedTP:
         T, N = a.shape[0], w.shape[0]
         # `out` is only a shape / stride carrier: the kernel stores through the push pointers
         dummy = self.region.tensor(self.off_gather[par] + self.rank * self.buf_bytes, (T, N), torch.bfloat16)
-        ops._gemm_tiles(a, w, bias=bias, out=dummy)   # the kernels that know the push epilogue
+        ops.gemm(a, w, bias=bias, out=dummy)
         return T, N
 
     def reduce_pushed(self, T, H, residual, norm_w, eps, w_offset=0.0):
