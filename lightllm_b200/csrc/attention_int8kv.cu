@@ -695,7 +695,9 @@ gqa_decode_q8_regs_kernel(const bf16* __restrict__ q, int64_t q_stride, const in
       }
       l_run[r] = l_run[r] * alpha[r] + rs;
     }
-    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {  // the maxima settle after a few tiles
+    // The maxima settle after a few tiles, and this kernel is bound by instructions: 37 requests of long contexts, fp8 pool, with this and
+    // the direct conversions 2078 -> 1921 us a step
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
       for (int nt = 0; nt < 16; ++nt) {
         o[nt][0] *= alpha[0];
