@@ -50,10 +50,10 @@ struct Params {
   int64_t out_stride;
   float scale_log2;
   int Hq, Hkv, pairs;  // pairs: the two query tiles are heads 2 y and 2 y + 1 (else tokens 0..127 and 128..255 of head y)
+  int n_slots;  // rows of the pool slice, or of the expanded matrix
   // paged
   const int *req_to_token, *b_req_idx;
   int64_t r2t_stride;
-  int n_slots;
   // expanded
   const int *cu_kv, *kv_start;
   int own, shared_col;
@@ -69,7 +69,7 @@ __device__ __forceinline__ float ex2_fast(float x) {  // 2^x, one MUFU instructi
 template <int DK, int DV, int BN, bool PAGED, bool SPLIT_P>
 __global__ void __launch_bounds__(THREADS, 1)
 prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
-                  const __grid_constant__ CUtensorMap tmShared, const Params p) {
+                  const __grid_constant__ CUtensorMap tmShared, const __grid_constant__ CUtensorMap tmRow, const Params p) {
   using L = Layout<DK, DV, BN>;
   static_assert(!SPLIT_P || BN == 64, "the two parts of the weights take the place of the scores");
   constexpr int KS = L::K_SLOTS, VS = L::V_SLOTS;
@@ -178,7 +178,9 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         __syncwarp();
       }
     } else if (elect_one()) {
-      const int row0 = p.cu_kv[b];
+      // The rows behind a request's last one are its neighbour's first.  Their scores are masked, but a weight of 0 times a value that
+      // is not finite is not 0: the values of the tile that holds the end come row by row, zeros in the place of the others.
+      const int row0 = p.cu_kv[b], rows = ready + q_len - kv0;
       for (int j = 0; j < n; ++j) {
         const int ks = j % KS, vs = j % VS;
         if (!mbar_wait(k_empty(ks), ((j / KS) & 1) ^ 1, abort_flag, status, 71)) break;
@@ -191,10 +193,20 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
         if (!mbar_wait(v_empty(vs), ((j / VS) & 1) ^ 1, abort_flag, status, 72)) break;
         mbar_expect_tx(v_full(vs), L::V_BYTES);
+        const uint32_t v = smem_base + L::OFF_V + vs * L::V_BYTES;
+        const int v_col = p.Hq * p.own + y * DV;
+        if ((j + 1) * BN <= rows) {
 #pragma unroll
-        for (int c = 0; c < DV / 64; ++c)
-          tma_load_2d(smem_base + L::OFF_V + vs * L::V_BYTES + c * BN * 128, &tmKV, v_full(vs), p.Hq * p.own + y * DV + c * 64,
-                      row0 + j * BN);
+          for (int c = 0; c < DV / 64; ++c) tma_load_2d(v + c * BN * 128, &tmKV, v_full(vs), v_col + c * 64, row0 + j * BN);
+        } else {
+#pragma unroll 1
+          for (int i = j * BN; i < (j + 1) * BN; i += 4) {
+            auto row = [&](int e) { return i + e < rows ? row0 + i + e : p.n_slots; };  // row n_slots: out of range, reads zeros
+#pragma unroll
+            for (int c = 0; c < DV / 64; ++c)
+              tma_gather4(v + c * BN * 128 + (i - j * BN) * 128, &tmRow, v_full(vs), v_col + c * 64, row(0), row(1), row(2), row(3));
+          }
+        }
       }
     }
     __syncwarp();
@@ -364,8 +376,8 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }
 
 template <int DK, int DV, int BN, bool PAGED, bool SPLIT_P>
-int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ts, const Params& p, int B, int max_q_len,
-              cudaStream_t st) {
+int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& ts, const CUtensorMap& trow, const Params& p, int B,
+              int max_q_len, cudaStream_t st) {
   using L = Layout<DK, DV, BN>;
   static_assert(L::BYTES <= 227 * 1024, "shared memory");
   static_assert(2 * BN + 2 * DV <= 512, "tensor memory");
@@ -379,7 +391,7 @@ int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& 
   }
   const int rows = p.pairs ? BM : 2 * BM;
   prefill_fa_kernel<DK, DV, BN, PAGED, SPLIT_P>
-      <<<dim3(p.pairs ? p.Hq / 2 : p.Hq, B, cdiv(max_q_len, rows)), THREADS, L::BYTES, st>>>(tq, tkv, ts, p);
+      <<<dim3(p.pairs ? p.Hq / 2 : p.Hq, B, cdiv(max_q_len, rows)), THREADS, L::BYTES, st>>>(tq, tkv, ts, trow, p);
   LLB_LAUNCH_CHECK();
   return LLB_OK;
 }
@@ -410,7 +422,7 @@ LLB_EXPORT int llb_gqa_prefill_fa(const void* q, int64_t q_stride, int T, const 
   p.cu_q = cu_q, p.b_ready_len = b_ready_len, p.out = (bf16*)out, p.out_stride = out_stride, p.scale_log2 = sm_scale * kLog2e;
   p.Hq = Hq, p.Hkv = Hkv, p.pairs = (Hq / Hkv) % 2 == 0;
   p.req_to_token = req_to_token, p.b_req_idx = b_req_idx, p.r2t_stride = r2t_stride, p.n_slots = n_slots;
-  return launch_fa<128, 128, 128, true, false>(tq, tkv, tkv, p, B, max_q_len, st);
+  return launch_fa<128, 128, 128, true, false>(tq, tkv, tkv, tkv, p, B, max_q_len, st);
 }
 
 // q [T, >= H * 192] bf16 (row pitch q_stride), kv [kv_rows, H * own | H * dv] (pitch kv_stride), out [T, >= H * dv].  Request b's
@@ -424,10 +436,12 @@ LLB_EXPORT int llb_latent_prefill_fa(const void* q, int64_t q_stride, const void
   if (!(sm_scale > 0.f) || H <= 0 || kv_rows <= 0 || (out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
   if (B > 65535 || cdiv(max_q_len, BM) > 65535 || (dv != 64 && dv != 128) || (own != 128 && own != 192)) return LLB_ERR_UNSUPPORTED;
   if (own == 128 && (shared == nullptr || shared_col < 0 || (shared_col % 8))) return LLB_ERR_BAD_ARG;
-  CUtensorMap tq, tkv, ts;
+  CUtensorMap tq, tkv, ts, trow;
   int rc = make_tmap_2d(&tq, q, 2, (uint64_t)T, (uint64_t)H * 192, (uint64_t)q_stride, BM, 64);
   if (rc) return rc;
   rc = make_tmap_2d(&tkv, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (own + dv), (uint64_t)kv_stride, 64, 64);
+  if (rc) return rc;
+  rc = make_tmap_2d(&trow, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (own + dv), (uint64_t)kv_stride, 1, 64);
   if (rc) return rc;
   ts = tkv;
   if (own == 128) {
@@ -437,7 +451,7 @@ LLB_EXPORT int llb_latent_prefill_fa(const void* q, int64_t q_stride, const void
   Params p;
   memset(&p, 0, sizeof(p));
   p.cu_q = cu_q, p.b_ready_len = b_ready_len, p.out = (bf16*)out, p.out_stride = out_stride, p.scale_log2 = sm_scale * kLog2e;
-  p.Hq = p.Hkv = H, p.cu_kv = cu_kv, p.kv_start = kv_start, p.own = own, p.shared_col = shared_col;
-  return dv == 64 ? launch_fa<192, 64, 64, false, true>(tq, tkv, ts, p, B, max_q_len, st)
-                  : launch_fa<192, 128, 64, false, true>(tq, tkv, ts, p, B, max_q_len, st);
+  p.Hq = p.Hkv = H, p.n_slots = kv_rows, p.cu_kv = cu_kv, p.kv_start = kv_start, p.own = own, p.shared_col = shared_col;
+  return dv == 64 ? launch_fa<192, 64, 64, false, true>(tq, tkv, ts, trow, p, B, max_q_len, st)
+                  : launch_fa<192, 128, 64, false, true>(tq, tkv, ts, trow, p, B, max_q_len, st);
 }

@@ -46,6 +46,32 @@ def test_expanded_attention(new, ready, dv):
     assert (out.float() - want).abs().max().item() < 2e-2
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("new,ready", [([1, 100], [0, 0]), ([63, 1], [0, 64]), ([64, 64], [1, 0]), ([130, 70], [255, 3])])
+def test_a_request_does_not_see_its_neighbour(new, ready, bad):
+    """Keys and values of the requests lie back to back; the first one's output is what it is alone, whatever the second one holds."""
+    H, own, rope, lat, dv = 3, 128, 64, 512, 128
+    g = torch.Generator(device="cuda").manual_seed(5)
+    first, rows, T = new[0] + ready[0], sum(new) + sum(ready), sum(new)
+    q = torch.randn(T, H * (own + rope), device="cuda", generator=g).bfloat16()
+    kv = torch.randn(rows, H * (own + dv), device="cuda", generator=g).bfloat16()
+    c = torch.randn(rows, lat + rope, device="cuda", generator=g).bfloat16()
+    kv[first:], c[first:] = bad, bad
+
+    def run(n):
+        t, r = sum(new[:n]), sum(new[:n]) + sum(ready[:n])
+        cu = torch.tensor([0] + torch.tensor(new[:n]).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+        kr = mla.KeyRange(torch.tensor(ready[:n]), torch.tensor(new[:n]), 0, "cuda")
+        out = torch.empty((t, H * dv), device="cuda", dtype=torch.bfloat16)
+        mla.latent_prefill(q[:t], kv[:r], c[:r], lat, own, H, own + rope, dv, cu, torch.tensor(ready[:n], dtype=torch.int32, device="cuda"),
+                           kr, max(new[:n]), 0.1, out)
+        return out[: new[0]]
+
+    alone = run(1)
+    assert alone.isfinite().all() and torch.equal(run(2), alone)
+
+
 def test_rule(monkeypatch):
     t = torch.tensor
     row = 128 * 256 * 2
