@@ -11,14 +11,16 @@
 //          as the sum of two bf16 values, which makes up for the rounding of the expanded keys and values)
 //   O_t += P_t . V       A operand from tensor memory, accumulated there over all key tiles
 // One thread issues all MMAs in the order  P0.V, Q0.K', P1.V, Q1.K'  so that the tensor core works on one query tile while the
-// softmax warps work on the other.  The running maximum that the weights refer to moves only when a row's maximum has grown by more
-// than 2^8 (the weights stay below 2^8 and keep their relative precision); only then is O, read-multiply-write, rescaled.
+// softmax warps work on the other.  O is rescaled, read-multiply-write, when a row's maximum has grown: at once where the weights are
+// single bf16 values, so that the weight of the largest key is exactly 1 (with a slack of 2^8 it is rounded like the others, and the error
+// against 64 bits grew from 0.0018 to 0.0023 for 1000 keys with scores of spread 2.5); by more than 2^8 where they are the sum of two.
 //
 // What bounds it: per 128 x 128 scores of head size 128, 1024 cycles of MMA and 1024 of exponentials (16 a cycle); it takes about 2100
-// (cycle counters: softmax 2300 per query tile and key tile, half of it hidden).  The kernel that was here (attention_tc.cu: one query
-// tile, P through shared memory, O in registers, K/V gathered by two warps with 16-byte copies, and every MMA's operands moved to
-// uniform registers, see elect_one) needed about 10000.  B200, 32 query and 8 KV heads: 16 x 1024 tokens 746 -> 237 us; six ragged pieces
-// of up to 2900 tokens behind up to 6000 1319 -> 490 us; 8192 tokens 540 us (1.02 PFLOP/s).
+// (cycle counters without rescaling: softmax 2300 per query tile and key tile, half of it hidden; a warp rescales 128 columns when one of
+// its rows' maxima grew).  attention_tc.cu (one query tile, P through shared memory, O in registers, K/V gathered by two warps with 16-byte
+// copies, and every MMA's operands moved to uniform registers, see elect_one) needs about 10000.  B200, 32 query and 8 KV heads, scores of
+// spread 2, kernel alone at burst clocks: 16 x 1024 tokens 248 us, 8192 tokens 605 us, 4 x 2048 with 4 KV heads 195 us (229, 543 and 178
+// with a slack of 2^8; 16 x 1024 took attention_tc.cu 746).
 #include "sm100_ptx.cuh"
 
 using namespace llb;
@@ -31,7 +33,7 @@ constexpr int BM = 128;
 constexpr int THREADS = 12 * 32;  // warp 0: Q and K/V loads (paged: with warps 2, 3), warp 1: MMA, warps 4..7 / 8..11: softmax of query
                                   // tile 0 / 1
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kSlack = 8.f;     // log2 of the largest weight before the maximum is moved
+constexpr float kSlack = 8.f;     // SPLIT_P: log2 of the largest weight before the maximum is moved
 
 __device__ int g_attn_fa_status = 0;
 
@@ -289,7 +291,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
         for (int c = 0; c < BN; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(s[c]));
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
-        const bool moved = top > m + kSlack || m == -INFINITY;
+        const bool moved = top > m + (SPLIT_P ? kSlack : 0.f) || m == -INFINITY;
         if (__any_sync(0xffffffffu, moved)) {
           const float m_new = moved ? fmaxf(m, top) : m;
           if (j > 0) {  // O holds the tiles before this one
@@ -297,16 +299,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             l *= alpha;
             mbar_wait(o_full(t), (j - 1) & 1, abort_flag, status, 78);
             tc_fence_after();
-#pragma unroll 1
-            for (int c = 0; c < DV; c += 32) {
-              uint32_t r[32];
-              tmem_ld_32x32(t_o + c, r);
-              tmem_wait_ld_of(r);
-              tmem_wait_ld_of(r + 16);
-#pragma unroll
-              for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
-              tmem_st_32x32(t_o + c, r);
-            }
+            tmem_scale<DV>(t_o, alpha);
           }
           m = m_new;
         }

@@ -9,11 +9,11 @@
 //   P  = exp2(S - m), one thread per head, written as bf16 over the scores
 //   O += P . V     V is the CTA's half of the key tile itself, read as an MN-major operand
 // The scores of the next tile are issued before the weights of the current one are waited for.  Tiles of 64 pool rows come by TMA
-// gathers through the slot table, two in flight.  The maximum moves as in attention_fa.cu.
+// gathers through the slot table, two in flight.  The output is rescaled whenever a head's maximum grows, as in attention_fa.cu.
 //
 // What bounds it: 1152 cycles of MMA for the scores of a tile (64 keys: as many as the 16 KB of Q per 16 columns take to read) and 512
-// for P . V, against 72 KB per tile from L2.  B200, us, mla.cu / here: 96 requests of 1025 to 2048 positions, 128 heads 755 / 166; one of
-// 1500 104 / 20; 128 of 1100, 32 heads 206 / 120; 96 of 1025 to 2048, 16 heads 176 / 159, 8 heads 172 / 158.
+// for P . V, against 72 KB per tile from L2.  B200, us, mla.cu / here: 96 requests of 1025 to 2048 positions, 128 heads 747 / 176, 64
+// 435 / 173, 32 285 / 173, 16 182 / 169, 8 181 / 166.
 #include "sm100_ptx.cuh"
 
 using namespace llb;
@@ -32,7 +32,6 @@ constexpr int S_COL = 0, Q_COL = 128, O_COL = 256;     // tensor memory: S0 | S1
 constexpr int LOADERS = 8;                             // a gather costs its warp about 70 cycles to issue, and a tile has 144
 constexpr int THREADS = (5 + LOADERS) * 32;            // warp 0 and 6 ..: loads, warp 1: MMA, warps 2..5: softmax
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kSlack = 8.f;
 
 struct Params {
   const bf16* q_lat;  // [T, H, 512]
@@ -216,7 +215,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
       for (int c = 0; c < BN; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(s[c]));
       const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
-      const bool moved = top > m + kSlack || m == -INFINITY;
+      const bool moved = top > m || m == -INFINITY;
       if (__any_sync(0xffffffffu, moved)) {
         const float m_new = moved ? fmaxf(m, top) : m;
         if (j > 0) {  // O holds the tiles before this one
@@ -224,16 +223,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           l *= alpha;
           mbar_wait(o_full, (j - 1) & 1, abort_flag, p.status, 87);  // s_full of tile j came after P . V of tile j - 2: one phase behind
           tc_fence_after();
-#pragma unroll 1
-          for (int c = 0; c < 256; c += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32(t_lane + O_COL + c, r);
-            tmem_wait_ld_of(r);
-            tmem_wait_ld_of(r + 16);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
-            tmem_st_32x32(t_lane + O_COL + c, r);
-          }
+          tmem_scale<256>(t_lane + O_COL, alpha);
         }
         m = m_new;
       }

@@ -236,6 +236,21 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t* r)
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// COLS fp32 columns of the warp's 32 lanes times a factor per lane.  Not unrolled: with two blocks of columns in flight the prompt kernel
+// spilt registers and took 17 % longer.
+template <int COLS>
+__device__ __forceinline__ void tmem_scale(uint32_t taddr, float f) {
+#pragma unroll 1
+  for (int c = 0; c < COLS; c += 32) {
+    uint32_t r[32];
+    tmem_ld_32x32(taddr + c, r);
+    tmem_wait_ld_of(r);
+    tmem_wait_ld_of(r + 16);
+#pragma unroll
+    for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * f);
+    tmem_st_32x32(taddr + c, r);
+  }
+}
 __device__ __forceinline__ void umma_fp8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(

@@ -71,3 +71,25 @@ def test_one_warp_rescales(B, first):
     assert (outs[0].double() - want).abs().max().item() < 2e-2   # weights and outputs (up to 1.8) rounded to bf16
     assert all(torch.equal(outs[0], o) for o in outs)
     assert int(ops.gemm_status("cuda:0").item()) == 0
+
+
+@pytest.mark.parametrize("keys,spread", [(300, 2.5), (300, 4.0), (1000, 2.5), (200, 1.0)])
+def test_error_of_sharp_scores(keys, spread, monkeypatch):
+    """As for prompt attention: the error against 64 bits is that of a pass in 64 bits with an exact running maximum."""
+    from test_gpu_prompt_attention import running_softmax
+
+    monkeypatch.setattr(mla, "mla_decode_splits", lambda *a: 1)
+    B, h = 8, 128
+    g = torch.Generator(device="cuda").manual_seed(keys)
+    kv = torch.randn(B * keys, 1, 576, device="cuda", generator=g).to(BF)
+    q = (torch.randn(B, h, 576, device="cuda", generator=g) * spread).to(BF)
+    q_lat, q3 = q[:, :, :512].contiguous(), torch.nn.functional.pad(q[:, :, 512:], (128, 0))
+    r2t = torch.arange(B * keys, dtype=torch.int32, device="cuda").view(B, keys)
+    i = torch.arange(B + 1, dtype=torch.int32, device="cuda")
+    seq = torch.full((B,), keys, dtype=torch.int32, device="cuda")
+    got = mla.mla_attention(q_lat, q3[:, :, 128:], kv, r2t, i[:B], seq, i, seq - 1, 512, 576 ** -0.5, False, 1, keys)
+    rows = kv.view(B, keys, 576).double()
+    s = q.double() @ rows.transpose(1, 2) * 576 ** -0.5
+    want = torch.softmax(s, -1) @ rows[:, :, :512]
+    err = lambda x: ((x - want).norm() / want.norm()).item()  # noqa: E731
+    assert err(got.double()) <= 1.05 * err(running_softmax(s, rows[:, :, :512], 64).float().to(BF).double())
