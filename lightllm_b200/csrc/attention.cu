@@ -47,7 +47,7 @@ __device__ __forceinline__ float gate_factor(const OutGate& g, int b, int h, int
   return p == nullptr ? g.scale : g.scale / (1.f + __expf(-__bfloat162float(p[b * g.stride + (g.elem ? h * DV + d : h)])));
 }
 
-template <int DK, int DV, int STAGES, bool SPLIT_P>
+template <int DK, int DV, int STAGES, bool SPLIT_P, bool MANY>
 __global__ void __launch_bounds__(128)
 gqa_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const bf16* __restrict__ kv_layer,
                   const int* __restrict__ req_to_token, int64_t r2t_stride, const int* __restrict__ b_req_idx,
@@ -347,8 +347,7 @@ gqa_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const bf16* __re
 
   if (!SPLIT_P && shares > 0) {
     __shared__ int start[SPLIT_P ? 1 : kMaxShareBatch + 1];
-    const int share = decode_shares(b_seq_len, B, shares, num_splits, start);
-    for_each_share(start, B, share, blockIdx.x, [&](int b, int slot, int count, int tile0, int tile1) {
+    for_each_share<MANY>(b_seq_len, B, shares, num_splits, blockIdx.x, start, [&](int b, int slot, int count, int tile0, int tile1) {
       work(b, slot, count, tile0, tile1);
       __syncthreads();  // the rings and the merge buffers are free again
     });
@@ -589,23 +588,33 @@ int set_smem(K kernel, int bytes) {
 
 }  // namespace
 
-// Number of KV splits the decode launcher will use for a batch (the caller sizes the
-// scratch buffers with it): enough CTAs to fill the GPU, at least 256 tokens per split.
-// The most CTAs that work on one request's context (slots of partial results per request; 1: no merge).  With `w` of them for a
-// request of average length the GPU is full (four CTAs per SM wanted); a long one may get 4 w (see decode_shares).  A batch that fills
-// the GPU twice over runs unsplit.
+// Partial results per request of a decode launch that cuts every context into the same number of equal parts: enough CTAs to fill the
+// GPU (four per SM wanted), at least 256 tokens per part.
 constexpr int kDecodeCtas = 148 * 4;
+LLB_EXPORT int llb_gqa_decode_equal_parts(int B, int Hq, int Hkv, int max_seq_len) {
+  const int ctas = B * Hkv * cdiv(Hq / Hkv, 16);
+  const int want = cdiv(kDecodeCtas, ctas), cap = max_seq_len > 0 ? cdiv(max_seq_len, 256) : 1;
+  const int s = want < cap ? want : cap;
+  return s < 64 ? s : 64;
+}
+// Whether a launch shares the batch out over one wave of CTAs (for_each_share) instead.  Equal parts that all run at once are as good
+// without the prefix sum (2 requests of 4000 tokens, 4 KV heads 14.3 us in parts, 17.9 shared), and so are those of a single request,
+// which has no neighbour to be balanced against.
+static bool decode_shared(int B, int groups, int num_splits) {
+  return num_splits > 1 && B > 1 && B <= kMaxShareBatch && (int64_t)B * groups * num_splits > kDecodeCtas / 2;
+}
+// The most CTAs that work on one request's context (slots of partial results per request; 1: no merge).  In a launch that shares the
+// batch out a request of average length gets a quarter of them, a long one may get all.  Batches that fill the GPU anyway are not cut:
+// 100 requests of 125 to 1000 tokens, 8 KV heads 47.6 us unsplit, 60.4 shared.
 LLB_EXPORT int llb_gqa_decode_num_splits(int B, int Hq, int Hkv, int max_seq_len) {
-  int G = Hq / Hkv;
-  int ctas = B * Hkv * ((G + 15) / 16);
-  if (ctas >= 2 * kDecodeCtas) return 1;
-  int want = 4 * ((kDecodeCtas + ctas - 1) / ctas);
-  int cap = (max_seq_len + 16 * kMinShareTiles - 1) / (16 * kMinShareTiles);
-  if (cap < 1) cap = 1;
-  int s = want < cap ? want : cap;
-  if (s < 1) s = 1;
-  if (s > 64) s = 64;
-  return s;
+  const int groups = Hkv * cdiv(Hq / Hkv, 16), parts = llb_gqa_decode_equal_parts(B, Hq, Hkv, max_seq_len);
+  if (B == 1) {  // one wave of two CTAs per SM: 12000 tokens 24.6 us with 47 parts, 18 with 37
+    const int wave = kDecodeCtas / 2 > groups ? kDecodeCtas / 2 / groups : 1;
+    return parts < wave ? parts : wave;
+  }
+  if (!decode_shared(B, groups, parts)) return parts;
+  const int slots = 4 * cdiv(kDecodeCtas, B * groups), cap = cdiv(max_seq_len, 16 * kMinShareTiles), s = slots < cap ? slots : cap;
+  return s < 64 ? s : 64;
 }
 
 template <int DK, int DV, bool SPLIT_P>
@@ -617,15 +626,18 @@ static int launch_decode(const void* q, int64_t q_stride, const void* kv_layer, 
   const int G = Hq / Hkv;
   const int groups = Hkv * ((G + 15) / 16);
   // Shares of equal length, one wave of two CTAs per SM (100 KB of rings each)
-  const int shares = !SPLIT_P && num_splits > 1 && B <= kMaxShareBatch ? (kDecodeCtas / 2 > groups ? kDecodeCtas / 2 / groups : 1) : 0;
-  const dim3 grid = shares > 0 ? dim3(shares, groups, 1) : dim3(num_splits, groups, B);
-  static DeviceOnce configured;
-  if (!configured.done()) {
-    int rc = set_smem(gqa_decode_kernel<DK, DV, STAGES, SPLIT_P>, decode_smem_bytes<DK, DV>());
+  const int shares = !SPLIT_P && decode_shared(B, groups, num_splits) ? (kDecodeCtas / 2 > groups ? kDecodeCtas / 2 / groups : 1) : 0;
+  const bool many = shares > 0 && 2 * B > shares;
+  const dim3 grid = shares > 0 ? dim3(many && B > shares ? B : shares, groups, 1) : dim3(num_splits, groups, B);
+  auto kernel = gqa_decode_kernel<DK, DV, STAGES, SPLIT_P, false>;
+  if (!SPLIT_P && many) kernel = gqa_decode_kernel<DK, DV, STAGES, SPLIT_P, !SPLIT_P>;
+  static DeviceOnce configured[2];
+  if (!configured[many].done()) {
+    int rc = set_smem(kernel, decode_smem_bytes<DK, DV>());
     if (rc) return rc;
-    configured.set();
+    configured[many].set();
   }
-  launch_pdl(gqa_decode_kernel<DK, DV, STAGES, SPLIT_P>, grid, dim3(128), decode_smem_bytes<DK, DV>(), st, (const bf16*)q,
+  launch_pdl(kernel, grid, dim3(128), decode_smem_bytes<DK, DV>(), st, (const bf16*)q,
              q_stride, (const bf16*)kv_layer, req_to_token, r2t_stride, b_req_idx, b_seq_len, (bf16*)out, out_stride, part_o,
              part_lse, Hq, Hkv, num_splits, B, shares, sm_scale * kLog2e, rule, gate);
   LLB_LAUNCH_CHECK();

@@ -494,7 +494,7 @@ __device__ __forceinline__ uint32_t cvt_v_pair(uint32_t a, uint32_t b, int i) {
   }
 }
 
-template <bool FP8>
+template <bool FP8, bool MANY>
 __global__ void __launch_bounds__(128)
 gqa_decode_q8_regs_kernel(const bf16* __restrict__ q, int64_t q_stride, const int8_t* __restrict__ kv_layer,
                           const int* __restrict__ req_to_token, int64_t r2t_stride, const int* __restrict__ b_req_idx,
@@ -783,8 +783,7 @@ gqa_decode_q8_regs_kernel(const bf16* __restrict__ q, int64_t q_stride, const in
 
   if (shares > 0) {
     __shared__ int start[kMaxShareBatch + 1];
-    const int share = decode_shares(b_seq_len, B, shares, num_splits, start);
-    for_each_share(start, B, share, blockIdx.x, [&](int b, int slot, int count, int tile0, int tile1) {
+    for_each_share<MANY>(b_seq_len, B, shares, num_splits, blockIdx.x, start, [&](int b, int slot, int count, int tile0, int tile1) {
       work(b, slot, count, tile0, tile1);
       __syncthreads();  // the rings and the merge buffers are free again
     });
@@ -886,17 +885,18 @@ int launch_decode8(const void* q, int64_t q_stride, const void* kv_layer, const 
     }                                                                                                               \
   }
   if (D == 128 && kv8_regs_enabled()) {
-    static DeviceOnce configured;     
-    if (!configured.done()) {
-      cudaError_t e = cudaFuncSetAttribute(gqa_decode_q8_regs_kernel<FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kRegSmemBytes);
-      if (e != cudaSuccess) return (int)e;
-      configured.set();  
-    }
     // shares of equal length, one wave of three CTAs per SM (registers, 72 KB of rings each)
     const int groups = Hkv * ((G + 15) / 16), ctas = 148 * 3;
-    const int shares = num_splits > 1 && B <= kMaxShareBatch ? (ctas > groups ? ctas / groups : 1) : 0;
-    launch_pdl(gqa_decode_q8_regs_kernel<FP8>, shares > 0 ? dim3(shares, groups, 1) : grid, dim3(128), kRegSmemBytes, st,
+    const int shares = num_splits > 1 && B > 1 && B <= kMaxShareBatch && (int64_t)B * groups * num_splits > ctas ? (ctas > groups ? ctas / groups : 1) : 0;
+    const bool many = shares > 0 && 2 * B > shares;
+    auto kernel = many ? gqa_decode_q8_regs_kernel<FP8, true> : gqa_decode_q8_regs_kernel<FP8, false>;
+    static DeviceOnce configured[2];
+    if (!configured[many].done()) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemBytes);
+      if (e != cudaSuccess) return (int)e;
+      configured[many].set();
+    }
+    launch_pdl(kernel, shares > 0 ? dim3(many && B > shares ? B : shares, groups, 1) : grid, dim3(128), kRegSmemBytes, st,
                (const bf16*)q, q_stride, (const int8_t*)kv_layer, req_to_token, r2t_stride, b_req_idx, b_seq_len, (bf16*)out,
                out_stride, part_o, part_lse, Hq, Hkv, num_splits, B, shares, sl2, head_scales);
     LLB_LAUNCH_CHECK();

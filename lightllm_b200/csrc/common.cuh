@@ -206,15 +206,23 @@ struct KeyRule {
     return chunk > 0 ? p - p % chunk : 0;
   }
 };
-// Work of a decode step whose contexts are cut into shares of equal length over the whole batch: the 16-token tiles of all requests
-// lie back to back, CTA `cta` of `ctas` takes tiles [cta * share, (cta + 1) * share), which may end one request and begin others.
-// With the same number of shares per request instead, ragged contexts make the longest one's shares last several times the mean,
-// and a grid of more CTAs than fit at once ends in a wave that is nearly empty.  A share has at least kMinShareTiles, and no
-// request touches more than `cap` CTAs (the slots of its partial results).  start [B + 1] (shared): first tile of each request; every
-// request has at least one.  Every CTA does the same prefix sum over the lengths (B loads, served by L2); 128 threads, all take part.
+// Work of a decode step whose contexts are cut into shares over the whole batch: the 16-token tiles of all requests lie back to back, CTA
+// `cta` of `ctas` takes tiles [cta * share, (cta + 1) * share), which may end one request and begin others.  With the same number of
+// shares per request instead, ragged contexts make the longest one's shares last several times the mean, and a grid of more CTAs than
+// fit at once ends in a wave that is nearly empty.  A share has at least kMinShareTiles, and no request touches more than `cap` CTAs
+// (the slots of its partial results).  Short contexts are not worth that: a CTA that works on several of them one after the other
+// takes longer than one for each, so
+//   * where every request can have ctas / B CTAs of its own with at most 2 kMinShareTiles each, it gets them (8 requests of 37 to 300
+//     tokens, 8 KV heads: 16.9 us shared, 12.3 so)
+//   * MANY (2 B > ctas): where the contexts are short, requests are not cut; the grid has a CTA for each request (150 requests of 87 to
+//     700 tokens, 2 KV heads: 33.8 us shared, 25.6 so).  An instance of its own: the rules in one kernel cost the other one 5 us
+// start [B + 1] (shared): first tile of each request; every request has at least one.  Every CTA does the same prefix sum over the
+// lengths (B loads, served by L2); 128 threads, all take part.  Runs body(b, slot, slots, first tile, end tile) for every request that
+// the CTA works on; slot: which of the request's `slots` CTAs.
 constexpr int kMinShareTiles = 8;
 constexpr int kMaxShareBatch = 592;
-__device__ __forceinline__ int decode_shares(const int* __restrict__ seq_len, int B, int ctas, int cap, int* start) {
+template <bool MANY, typename Body>
+__device__ __forceinline__ void for_each_share(const int* __restrict__ seq_len, int B, int ctas, int cap, int cta, int* start, Body body) {
   __shared__ int sums[4], longest[4];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int each = (B + 127) / 128, b0 = t * each < B ? t * each : B, b1 = b0 + each < B ? b0 + each : B;
@@ -234,6 +242,19 @@ __device__ __forceinline__ int decode_shares(const int* __restrict__ seq_len, in
   }
   if (lane == 31) sums[w] = upto, longest[w] = most;
   __syncthreads();
+  most = max(max(longest[0], longest[1]), max(longest[2], longest[3]));
+  const int own = MANY ? 1 : min(cap, ctas / B);  // CTAs of a request
+  const int total = sums[0] + sums[1] + sums[2] + sums[3];
+  // own > 0 always holds without MANY; the code that the compiler makes with the test is the faster one (8 requests of 1500 to 12000
+  // tokens, one KV head: 23.6 us, 28.7 without)
+  if (MANY ? most <= (total <= 5 * kMinShareTiles * ctas ? 6 : 2) * kMinShareTiles : own > 0 && most <= 2 * kMinShareTiles * own) {
+    const int b = cta / own, slot = cta - b * own;
+    if (b >= B) return;
+    const int tiles = start[b + 1], want = min(own, (tiles + kMinShareTiles - 1) / kMinShareTiles);
+    const int per = (tiles + want - 1) / want, slots = (tiles + per - 1) / per;
+    if (slot < slots) body(b, slot, slots, slot * per, min(tiles, (slot + 1) * per));
+    return;
+  }
   for (int i = 0; i < w; ++i) upto += sums[i];
   int at = upto - sum;
   if (t == 0) start[0] = 0;
@@ -242,15 +263,9 @@ __device__ __forceinline__ int decode_shares(const int* __restrict__ seq_len, in
     start[b + 1] = at;
   }
   __syncthreads();
-  const int total = sums[0] + sums[1] + sums[2] + sums[3];
-  most = max(max(longest[0], longest[1]), max(longest[2], longest[3]));
-  return max(max((total + ctas - 1) / ctas, kMinShareTiles), (most + cap - 2) / (cap - 1));
-}
-// Runs body(b, slot, slots, first tile, end tile) for every request that CTA `cta` works on; slot: which of the request's `slots` CTAs.
-template <typename Body>
-__device__ __forceinline__ void for_each_share(const int* start, int B, int share, int cta, Body body) {
+  const int share = max(max((total + ctas - 1) / ctas, kMinShareTiles), (most + cap - 2) / (cap - 1));
   int u = cta * share;
-  const int end = min(u + share, start[B]);
+  const int end = min(u + share, total);
   if (u >= end) return;
   int b = 0;
   for (int hi = B - 1; b < hi;) {

@@ -690,7 +690,7 @@ class TransformerLM:
         st = InferState(is_prefill=False, batch_size=B, num_tokens=B, max_kv_len=max_kv_len, max_q_len=1,
                         b_req_idx=b_req_idx, b_seq_len=b_seq_len, mem_index=mem_index)
         if self.device.type == "cuda":
-            st.decode_num_splits = num_splits or ops.gqa_decode_num_splits(B, self.hq, max(self.hkv, 1), max_kv_len)
+            st.decode_num_splits = num_splits or self._decode_splits(B, max_kv_len)
         return st
 
     def _decode_body(self, st: InferState) -> torch.Tensor:
@@ -703,9 +703,13 @@ class TransformerLM:
         h = self._layers_forward(h, st)
         return self._lm_head(h, normed=True) if st.extra.get("normed") else self._lm_head(h)
 
+    def _decode_splits(self, B: int, max_kv_len: int) -> int:
+        eight_bit = str(self.extra.get("kv_type") or "").lower().startswith(("int8kv", "fp8kv"))
+        return ops.gqa_decode_num_splits(B, self.hq, max(self.hkv, 1), max_kv_len, ops.kv_quant.decode_shares(eight_bit, self.head_dim))
+
     def _graph_decode_splits(self, bucket: int) -> int:
-        """Shares the decode attention of a captured step cuts every context into."""
-        return ops.gqa_decode_num_splits(bucket, self.hq, max(self.hkv, 1), self.graph_max_len_in_batch)
+        """Slots of partial results per request in the decode attention of a captured step."""
+        return self._decode_splits(bucket, self.graph_max_len_in_batch)
 
     def _capture_decode_graph(self, bucket: int) -> dict:
         dev = self.device

@@ -406,8 +406,11 @@ def _scratch(device, n_o: int, n_lse: int):
     return cur
 
 
-def gqa_decode_num_splits(B, Hq, Hkv, max_seq_len) -> int:
-    return int(kernels().llb_gqa_decode_num_splits(c_int(B), c_int(Hq), c_int(Hkv), c_int(max_seq_len)))
+def gqa_decode_num_splits(B, Hq, Hkv, max_seq_len, shares: bool = True) -> int:
+    """Slots of partial results per request.  shares False: for kernels that cut every context into that many equal parts
+    (`kv_quant.decode_shares`)."""
+    f = kernels().llb_gqa_decode_num_splits if shares else kernels().llb_gqa_decode_equal_parts
+    return int(f(c_int(B), c_int(Hq), c_int(Hkv), c_int(max_seq_len)))
 
 
 def gqa_decode(q, kv_layer, req_to_token, b_req_idx, b_seq_len, Hq, Hkv, D, max_seq_len: int, sm_scale=None,

@@ -21,6 +21,7 @@ fp8_static_per_tensor_quant_mem_manager.py, common/basemodel/attention/triton/in
 from __future__ import annotations
 
 import math
+import os
 from typing import Optional
 
 import torch
@@ -237,6 +238,13 @@ def rope_kv_scatter_(qkv, layer, cos, sin, pos, slot, Hq, Hkv, D, rot_dim=None, 
     return qkv
 
 
+def decode_shares(eight_bit: bool, D: int) -> bool:
+    """Whether decode attention shares a batch's tiles out over the CTAs.  The 8-bit kernel that widens its tiles in shared memory (head
+    size 64, or LLB_KV8_REGS=0) cuts every context into equal parts (B200, us, with the number of parts for it / four times as many: 64
+    requests of 1000 to 2000 tokens, 8 KV heads 53.8 / 65.0; 4 of 2000 to 4000 14.9 / 18.4)."""
+    return not eight_bit or D == 128 and os.environ.get("LLB_KV8_REGS", "1")[:1] != "0"
+
+
 def gqa_decode(q, layer, req_to_token, b_req_idx, b_seq_len, Hq, Hkv, D, max_seq_len, sm_scale=None,
                out=None, num_splits: Optional[int] = None, scratch=None):
     from . import _count, _scratch, c_int, check, f32, gqa_decode as plain, gqa_decode_num_splits, i64, kernels, ptr, \
@@ -258,7 +266,7 @@ def gqa_decode(q, layer, req_to_token, b_req_idx, b_seq_len, Hq, Hkv, D, max_seq
     if out is None:
         out = torch.empty((B, Hq, D), dtype=q.dtype, device=q.device)
     if num_splits is None:
-        num_splits = gqa_decode_num_splits(B, Hq, Hkv, max_seq_len)
+        num_splits = gqa_decode_num_splits(B, Hq, Hkv, max_seq_len, decode_shares(True, D))
     po = pl = None
     if num_splits > 1:
         po, pl = scratch if scratch is not None else _scratch(q.device, B * Hq * num_splits * D, B * Hq * num_splits)

@@ -79,3 +79,35 @@ def test_fused_store_is_the_separate_one(D, rot, kind, T, norm):
     ops.rope_kv_scatter_(q2, tmp, cos, sin, pos, torch.arange(T, dtype=torch.int32, device="cuda"), Hq, Hkv, D, rot, *nw)
     kv_quant.quant_store_(b, tmp, slot)
     assert torch.equal(q1, q2) and torch.equal(a.data, b.data)
+
+
+@pytest.mark.parametrize("lens", [[130] * 5, [256, 1, 17], list(range(16, 130, 4)), [2048, 3, 2047], [250] * 140 + [257] * 8, [255] * 147])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_short_contexts(lens, fp8):
+    """Batches whose requests get CTAs of their own, and their neighbours that are shared out."""
+    Hq, Hkv, D, B = 8, 2, 128, len(lens)
+    n, r2t, rows, b_len = _batch(lens)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    kv = torch.randn(n, 2 * Hkv, D, device="cuda", generator=g).to(BF)
+    q = torch.randn(B, Hq * D, device="cuda", generator=g).to(BF)
+    layer = kv
+    if fp8:
+        layer = kv_quant.Fp8KVLayer(torch.zeros(n, 2 * Hkv, D, dtype=torch.uint8, device="cuda"), D, torch.full((2 * Hkv,), 0.01, device="cuda"))
+        kv_quant.quant_store_(layer, kv, torch.arange(n, dtype=torch.int32, device="cuda"))
+        kv = layer.dequant_all(BF)
+    want = ref.gqa_decode(q.view(B, Hq, D).float(), kv.float(), r2t, rows, b_len, Hq, Hkv, D).view(B, Hq, D).float()
+    for splits in (2, 3, 17, 64):
+        got = ops.gqa_decode(q, layer, r2t, rows, b_len, Hq, Hkv, D, max(lens), num_splits=splits).float()
+        assert (got - want).abs().max().item() < 3e-2, splits   # as above
+
+
+def test_slots_of_partial_results():
+    """Kernels that cut every context into equal parts get the number of parts that fills the GPU, others four times as many slots; a batch
+    that fills the GPU by itself is not cut."""
+    equal = lambda b, h, n: max(1, min(-(-592 // (b * h)), -(-n // 256), 64))  # noqa: E731
+    for b, h, n in ((1, 8, 700), (4, 8, 4000), (64, 8, 2000), (74, 8, 2000), (100, 8, 1000), (592, 1, 5000), (600, 1, 300), (1183, 1, 9000)):
+        parts = equal(b, h, n)
+        assert ops.gqa_decode_num_splits(b, 4 * h, h, n, shares=False) == parts
+        slots = ops.gqa_decode_num_splits(b, 4 * h, h, n)
+        assert slots == 1 if parts == 1 else slots >= min(parts, 296 // h)
+    assert not kv_quant.decode_shares(True, 64) and kv_quant.decode_shares(True, 128) and kv_quant.decode_shares(False, 64)
