@@ -608,12 +608,10 @@ static bool decode_shared(int B, int groups, int num_splits) {
 // 100 requests of 125 to 1000 tokens, 8 KV heads 47.6 us unsplit, 60.4 shared.
 LLB_EXPORT int llb_gqa_decode_num_splits(int B, int Hq, int Hkv, int max_seq_len) {
   const int groups = Hkv * cdiv(Hq / Hkv, 16), parts = llb_gqa_decode_equal_parts(B, Hq, Hkv, max_seq_len);
-  if (B == 1) {  // one wave of two CTAs per SM: 12000 tokens 24.6 us with 47 parts, 18 with 37
-    const int wave = kDecodeCtas / 2 > groups ? kDecodeCtas / 2 / groups : 1;
-    return parts < wave ? parts : wave;
-  }
-  if (!decode_shared(B, groups, parts)) return parts;
-  const int slots = 4 * cdiv(kDecodeCtas, B * groups), cap = cdiv(max_seq_len, 16 * kMinShareTiles), s = slots < cap ? slots : cap;
+  if (parts == 1 || (B > 1 && !decode_shared(B, groups, parts))) return parts;
+  // one request: one wave of two CTAs per SM (12000 tokens 24.6 us with 47 parts, 21 with 37)
+  const int slots = B > 1 ? 4 * cdiv(kDecodeCtas, B * groups) : (kDecodeCtas / 2 > groups ? kDecodeCtas / 2 / groups : 1);
+  const int cap = max_seq_len > 0 ? cdiv(max_seq_len, 16 * kMinShareTiles) : 1, s = slots < cap ? slots : cap;
   return s < 64 ? s : 64;
 }
 
