@@ -220,7 +220,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       constexpr uint32_t IDESC_PV = umma_idesc(BM, 64, 1) | (1u << 16);  // B operand MN-major
       auto scores = [&](int t, int j) {
         const uint32_t q = smem_base + L::OFF_Q + t * L::Q_BYTES, k = smem_base + L::OFF_K + (j % KS) * L::K_BYTES;
-        mbar_wait(k_full(j % KS), (j / KS) & 1, abort_flag, status, 73);
+        if (!mbar_wait(k_full(j % KS), (j / KS) & 1, abort_flag, status, 73)) return false;
         tc_fence_after();
         const uint64_t dq = umma_smem_desc_sw128(q), dk = umma_smem_desc_sw128(k);  // offsets count 16-byte units
 #pragma unroll
@@ -228,11 +228,11 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           umma_bf16(tmem_base + L::S_COL + t * BN, dq + ((i >> 2) * BM * 8 + (i & 3) * 2), dk + ((i >> 2) * BN * 8 + (i & 3) * 2),
                     IDESC_S, i != 0);
         umma_commit(s_full(t));
+        return true;
       };
       auto values = [&](int t, int j) {
         const uint32_t v = smem_base + L::OFF_V + (j % VS) * L::V_BYTES;
-        mbar_wait(p_full(t), j & 1, abort_flag, status, 74);
-        mbar_wait(v_full(j % VS), (j / VS) & 1, abort_flag, status, 75);
+        if (!mbar_wait(p_full(t), j & 1, abort_flag, status, 74) || !mbar_wait(v_full(j % VS), (j / VS) & 1, abort_flag, status, 75)) return false;
         tc_fence_after();
         const uint64_t dv = umma_smem_desc_sw128_mn(v);
 #pragma unroll
@@ -242,22 +242,16 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             umma_bf16_ts(tmem_base + L::O_COL + t * DV + h * 64, tmem_base + L::S_COL + t * BN + i * 8,
                          dv + (h * BN * 8 + i % (BN / 16) * 128), IDESC_PV, (j | i) != 0);
         umma_commit(o_full(t));
+        return true;
       };
-      mbar_wait(q_full, 0, abort_flag, status, 76);
       // the second query tile sees at least the key tiles of the first, or has no rows
-      scores(0, 0);
-      if (n1 > 0) scores(1, 0);
-      umma_commit(k_empty(0));
-      for (int j = 0; j < n && !*abort_flag; ++j) {
+      bool ok = mbar_wait(q_full, 0, abort_flag, status, 76) && scores(0, 0) && (n1 == 0 || scores(1, 0));  // false: issue nothing more
+      if (ok) umma_commit(k_empty(0));
+      for (int j = 0; j < n && ok; ++j) {
         const bool k_next = j + 1 < n;
-        if (j < n0) {
-          values(0, j);
-          if (j + 1 < n0) scores(0, j + 1);
-        }
-        if (j < n1) {
-          values(1, j);
-          if (j + 1 < n1) scores(1, j + 1);
-        }
+        if (j < n0) ok = values(0, j) && (j + 1 >= n0 || scores(0, j + 1));
+        if (ok && j < n1) ok = values(1, j) && (j + 1 >= n1 || scores(1, j + 1));
+        if (!ok) break;
         umma_commit(v_empty(j % VS));
         if (k_next) umma_commit(k_empty((j + 1) % KS));
       }
@@ -274,7 +268,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const uint32_t t_s = t_lane + L::S_COL + t * BN, t_o = t_lane + L::O_COL + t * DV;
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < mine; ++j) {
-        mbar_wait(s_full(t), j & 1, abort_flag, status, 77);
+        if (!__all_sync(0xffffffffu, mbar_wait(s_full(t), j & 1, abort_flag, status, 77))) break;
         tc_fence_after();
         uint32_t s[BN];
 #pragma unroll
@@ -326,7 +320,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full(t));
       }
-      mbar_wait(o_full(t), (mine - 1) & 1, abort_flag, status, 79);
+      const bool whole = __all_sync(0xffffffffu, mbar_wait(o_full(t), (mine - 1) & 1, abort_flag, status, 79)) && !*abort_flag;
       tc_fence_after();
       // output: a warp parks its 32 rows in the (now idle) query tile and writes whole rows
       const float inv = l > 0.f ? 1.f / l : 0.f;
@@ -351,7 +345,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       for (int i = 0; i < CH; ++i) {
         const int id = i * 32 + lane, r = id / CH, ch = id % CH;
         const int tk = first_row(t) + lane_grp * 32 + r;
-        if (tk < q_len)
+        if (tk < q_len && whole)
           *reinterpret_cast<bf16x8*>(p.out + (int64_t)(q_begin + tk) * p.out_stride + head_of(t) * DV + ch * 8) =
               *reinterpret_cast<const bf16x8*>(stg + r * (DV * 2) + ((ch ^ (r & 7)) << 4));
       }

@@ -206,8 +206,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       uint32_t phase = 0;
       for (int i = 0; i < nk; ++i) {
         const int buf = FP8 ? i & 1 : 0;
-        if (FP8) mbar_wait(tempty_bar(buf), (((uint32_t)i >> 1) & 1u) ^ 1u, &abort_flag, p.status, 64);
-        mbar_wait(full_bar(stage), phase, &abort_flag, p.status, 62);
+        if (FP8 && !mbar_wait(tempty_bar(buf), (((uint32_t)i >> 1) & 1u) ^ 1u, &abort_flag, p.status, 64)) break;
+        if (!mbar_wait(full_bar(stage), phase, &abort_flag, p.status, 62)) break;
         tc_fence_after();
         const uint32_t sa = smem_base + stage * STAGE_BYTES;
         const uint64_t dw = umma_smem_desc_sw128(sa), dx = umma_smem_desc_sw128(sa + W_BYTES);
@@ -225,7 +225,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           phase ^= 1;
         }
       }
-      if (!FP8) umma_commit(tfull_bar(0));
+      if (!FP8) umma_commit(tfull_bar(0));  // also after a wait that ran out: the drain ends, and stores nothing
     }
     __syncwarp();
   } else if (warp < 2 + DRAIN) {
@@ -316,7 +316,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       if (s < splits) a.x += v[s].x, a.y += v[s].y, a.z += v[s].z, a.w += v[s].w;
     return a;
   };
-  for (uint32_t i = i0 + threadIdx.x; i < i1; i += THREADS) {
+  const bool aborted = *(volatile int*)&abort_flag != 0;
+  for (uint32_t i = i0 + threadIdx.x; i < i1 && !aborted; i += THREADS) {
     const uint32_t row = i / groups, g = i % groups;
     if (epi_gated(EPI)) {  // columns come as [32 gate | 32 up] pairs
       const uint32_t c = (g >> 3) * 64 + (g & 7) * 4;
@@ -366,7 +367,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       }
     }
   }
-  if (*(volatile int*)&abort_flag) settle_after_abort();
+  if (aborted) settle_after_abort();
   cluster_sync_all();  // nobody leaves while a peer may still read its share
   if (warp == 1) {
     tc_fence_after();

@@ -138,7 +138,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       constexpr uint32_t IDESC_PV = umma_idesc(128, 64, 1) | (1u << 16);  // B operand MN-major
       auto scores = [&](int j) {
         const uint32_t k = smem_base + OFF_K + (j & 1) * STAGE;
-        mbar_wait(full(j & 1), (j >> 1) & 1, abort_flag, p.status, 82);
+        if (!mbar_wait(full(j & 1), (j >> 1) & 1, abort_flag, p.status, 82)) return false;
         tc_fence_after();
         const uint32_t d = tmem_base + S_COL + (j & 1) * BN;
         const uint64_t dk = umma_smem_desc_sw128(k), dq = umma_smem_desc_sw128(smem_base);  // offsets count 16-byte units
@@ -151,13 +151,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             umma_bf16(d, dq + (((i - Q_TMEM / 16) >> 2) * (QBLOCK / 16) + (i & 3) * 2), kd, IDESC_S, 1);
         }
         umma_commit(s_full(j & 1));
+        return true;
       };
-      mbar_wait(q_full, 0, abort_flag, p.status, 83);
-      mbar_wait(qt_full, 0, abort_flag, p.status, 84);
+      const bool ready = mbar_wait(q_full, 0, abort_flag, p.status, 83) && mbar_wait(qt_full, 0, abort_flag, p.status, 84);
       tc_fence_after();
-      scores(0);
-      for (int j = 0; j < n; ++j) {
-        if (j + 1 < n) scores(j + 1);
+      const bool first = ready && scores(0);
+      for (int j = 0; j < n && first; ++j) {  // a wait that ran out: nothing more is issued
+        if (j + 1 < n && !scores(j + 1)) break;
         if (!mbar_wait(p_full(j & 1), (j >> 1) & 1, abort_flag, p.status, 85)) break;
         tc_fence_after();
         const uint32_t v = smem_base + OFF_K + (j & 1) * STAGE + half * 4 * BLOCK;
@@ -246,12 +246,12 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (lane == 0) mbar_arrive(p_full(j & 1));
     }
     // not o_full: the scores of the last tile were issued ahead of the last but one P . V, so o_full may be two phases behind here
-    mbar_wait(done, 0, abort_flag, p.status, 88);
+    const int valid = __all_sync(0xffffffffu, mbar_wait(done, 0, abort_flag, p.status, 88)) && !*abort_flag ? rows : 0;  // rows to store
     tc_fence_after();
     // output through the (now idle) query blocks: a warp parks 32 rows x 64 columns and writes whole lines
     const float inv = l > 0.f ? 1.f / l : 0.f;
     float* stg = reinterpret_cast<float*>(smem + lane_grp * (32 * 260));  // 32 rows x 65 floats
-    if (p.splits > 1 && half == 0 && row < rows)
+    if (p.splits > 1 && half == 0 && row < valid)
       p.part_lse[(qrow + row) * p.splits + split] = l > 0.f ? (m + log2f(l)) / kLog2e : -INFINITY;
 #pragma unroll 1
     for (int c = 0; c < 256; c += 64) {
@@ -268,7 +268,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int col = half * 256 + c + lane * 2;
       for (int r = 0; r < 32; ++r) {
         const int hr = lane_grp * 32 + r;
-        if (hr >= rows) break;
+        if (hr >= valid) break;
         const float x = stg[r * 65 + lane * 2], y = stg[r * 65 + lane * 2 + 1];
         if (p.splits == 1)
           *reinterpret_cast<uint32_t*>(p.out + (qrow + hr) * LAT + col) = pack_bf16x2(x, y);
