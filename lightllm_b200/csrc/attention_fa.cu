@@ -35,7 +35,7 @@ constexpr int THREADS = 12 * 32;  // warp 0: Q and K/V loads (paged: with warps 
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kSlack = 8.f;     // SPLIT_P: log2 of the largest weight before the maximum is moved
 
-__device__ int g_attn_fa_status = 0;
+__device__ int g_attn_fa_status = 0;  // a wait ran out in some launch, whatever word its caller gave
 
 template <int DK, int DV, int BN>
 struct Layout {
@@ -48,6 +48,7 @@ struct Layout {
 
 struct Params {
   const int *cu_q, *b_ready_len;
+  int* status;  // receives the code of a wait that ran out
   bf16* out;
   int64_t out_stride;
   float scale_log2;
@@ -88,7 +89,7 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const uint32_t q_full = bar + 8 * (2 * KS + 2 * VS + 6);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::OFF_BAR + 200);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::OFF_BAR + 204);
-  int* status = &g_attn_fa_status;
+  int* status = p.status;
 
   // heads fastest, late (long) query tiles first
   const int y = blockIdx.x, b = blockIdx.y;
@@ -97,7 +98,10 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
   if (q0 >= q_len) return;  // whole CTA: nothing allocated yet
   if (smem_base & 1023u) {
-    if (threadIdx.x == 0) atomicCAS(status, 0, 70);
+    if (threadIdx.x == 0) {
+      atomicCAS(status, 0, 70);
+      g_attn_fa_status = 70;
+    }
     return;
   }
   const int ready = p.b_ready_len[b];
@@ -355,7 +359,10 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) settle_after_abort();
+  if (*abort_flag) {
+    settle_after_abort();
+    if (threadIdx.x == 0) g_attn_fa_status = 1;
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
@@ -385,19 +392,21 @@ int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const CUtensorMap& 
 
 }  // namespace
 
-// 0 while every bounded wait of the kernel was met; 70: shared memory not where the layout needs it.
+// 0 while every bounded wait of the kernel was met; 70: shared memory not where the layout needs it; 1: a wait ran out (its code is in
+// the status word of that launch).
 LLB_EXPORT int llb_attn_fa_status() {
   int v = 0;
   cudaMemcpyFromSymbol(&v, g_attn_fa_status, sizeof(int));
   return v;
 }
 
-// Same contract as llb_gqa_prefill with head size 128; T rows of q, n_slots rows of the pool slice.
+// Same contract as llb_gqa_prefill with head size 128; T rows of q, n_slots rows of the pool slice; status: device int that receives the
+// code of a wait that ran out.
 LLB_EXPORT int llb_gqa_prefill_fa(const void* q, int64_t q_stride, int T, const void* kv_layer, int n_slots, const int* req_to_token,
                                   int64_t r2t_stride, const int* b_req_idx, const int* cu_q, const int* b_ready_len, void* out,
-                                  int64_t out_stride, int B, int max_q_len, int Hq, int Hkv, float sm_scale, cudaStream_t st) {
+                                  int64_t out_stride, int B, int max_q_len, int Hq, int Hkv, float sm_scale, int* status, cudaStream_t st) {
   if (B <= 0 || max_q_len <= 0 || T <= 0) return LLB_OK;
-  if (!(sm_scale > 0.f) || Hkv <= 0 || Hq % Hkv != 0 || n_slots <= 0 || (out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
+  if (!(sm_scale > 0.f) || status == nullptr || Hkv <= 0 || Hq % Hkv != 0 || n_slots <= 0 || (out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
   if (B > 65535 || cdiv(max_q_len, BM) > 65535) return LLB_ERR_UNSUPPORTED;
   CUtensorMap tq, tkv;
   int rc = make_tmap_2d(&tq, q, 2, (uint64_t)T, (uint64_t)Hq * 128, (uint64_t)q_stride, BM, 64);
@@ -406,7 +415,7 @@ LLB_EXPORT int llb_gqa_prefill_fa(const void* q, int64_t q_stride, int T, const 
   if (rc) return rc;
   Params p;
   memset(&p, 0, sizeof(p));
-  p.cu_q = cu_q, p.b_ready_len = b_ready_len, p.out = (bf16*)out, p.out_stride = out_stride, p.scale_log2 = sm_scale * kLog2e;
+  p.status = status, p.cu_q = cu_q, p.b_ready_len = b_ready_len, p.out = (bf16*)out, p.out_stride = out_stride, p.scale_log2 = sm_scale * kLog2e;
   p.Hq = Hq, p.Hkv = Hkv, p.pairs = (Hq / Hkv) % 2 == 0;
   p.req_to_token = req_to_token, p.b_req_idx = b_req_idx, p.r2t_stride = r2t_stride, p.n_slots = n_slots;
   return launch_fa<128, 128, 128, true, false>(tq, tkv, tkv, tkv, p, B, max_q_len, st);
@@ -418,9 +427,9 @@ LLB_EXPORT int llb_gqa_prefill_fa(const void* q, int64_t q_stride, int T, const 
 LLB_EXPORT int llb_latent_prefill_fa(const void* q, int64_t q_stride, const void* kv, int64_t kv_stride, int kv_rows,
                                      const void* shared, int64_t shared_stride, int shared_col, int own, const int* cu_q,
                                      const int* cu_kv, const int* kv_start, const int* b_ready_len, void* out, int64_t out_stride,
-                                     int B, int T, int max_q_len, int H, int dv, float sm_scale, cudaStream_t st) {
+                                     int B, int T, int max_q_len, int H, int dv, float sm_scale, int* status, cudaStream_t st) {
   if (B <= 0 || max_q_len <= 0 || T <= 0) return LLB_OK;
-  if (!(sm_scale > 0.f) || H <= 0 || kv_rows <= 0 || (out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
+  if (!(sm_scale > 0.f) || status == nullptr || H <= 0 || kv_rows <= 0 || (out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
   if (B > 65535 || cdiv(max_q_len, BM) > 65535 || (dv != 64 && dv != 128) || (own != 128 && own != 192)) return LLB_ERR_UNSUPPORTED;
   if (own == 128 && (shared == nullptr || shared_col < 0 || (shared_col % 8))) return LLB_ERR_BAD_ARG;
   CUtensorMap tq, tkv, ts, trow;
@@ -437,7 +446,7 @@ LLB_EXPORT int llb_latent_prefill_fa(const void* q, int64_t q_stride, const void
   }
   Params p;
   memset(&p, 0, sizeof(p));
-  p.cu_q = cu_q, p.b_ready_len = b_ready_len, p.out = (bf16*)out, p.out_stride = out_stride, p.scale_log2 = sm_scale * kLog2e;
+  p.status = status, p.cu_q = cu_q, p.b_ready_len = b_ready_len, p.out = (bf16*)out, p.out_stride = out_stride, p.scale_log2 = sm_scale * kLog2e;
   p.Hq = p.Hkv = H, p.n_slots = kv_rows, p.cu_kv = cu_kv, p.kv_start = kv_start, p.own = own, p.shared_col = shared_col;
   return dv == 64 ? launch_fa<192, 64, 64, false, true>(tq, tkv, ts, trow, p, B, max_q_len, st)
                   : launch_fa<192, 128, 64, false, true>(tq, tkv, ts, trow, p, B, max_q_len, st);

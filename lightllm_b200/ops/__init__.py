@@ -464,7 +464,7 @@ def gqa_prefill(q, kv_layer, req_to_token, b_req_idx, cu_q, b_ready_len, Hq, Hkv
         check(kernels().llb_gqa_prefill_fa(ptr(q), i64(q.stride(0)), c_int(T), ptr(kv_layer), c_int(kv_layer.shape[0]),
                                            ptr(req_to_token), i64(req_to_token.stride(0)), ptr(b_req_idx), ptr(cu_q),
                                            ptr(b_ready_len), ptr(out), i64(out.stride(0)), c_int(B), c_int(max_q_len), c_int(Hq),
-                                           c_int(Hkv), f32(scale), stream()), "gqa_prefill_fa")
+                                           c_int(Hkv), f32(scale), ptr(gemm_status(q.device)), stream()), "gqa_prefill_fa")
         _count()
         return out
     check(kernels().llb_gqa_prefill(ptr(q), i64(q.stride(0)), ptr(kv_layer), ptr(req_to_token),

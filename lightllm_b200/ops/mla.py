@@ -295,7 +295,8 @@ def latent_prefill(q, kv, c, col: int, own: int, H: int, dk: int, dv: int, cu_q,
     check(kernels().llb_latent_prefill_fa(ptr(q), i64(q.stride(0)), ptr(kv), i64(kv.stride(0)), c_int(kr.rows), ptr(c),
                                           i64(c.stride(0)), c_int(col), c_int(own), ptr(cu_q), ptr(kr.cu_kv), ptr(kr.kv_start),
                                           ptr(b_ready_len), ptr(out), i64(out.stride(0)), c_int(cu_q.shape[0] - 1),
-                                          c_int(q.shape[0]), c_int(max_q_len), c_int(H), c_int(dv), f32(scale), stream()),
+                                          c_int(q.shape[0]), c_int(max_q_len), c_int(H), c_int(dv), f32(scale),
+                                          ptr(gemm_status(q.device)), stream()),
           "latent_prefill_fa")
     _count()
     return out

@@ -92,5 +92,6 @@ def test_prefill_many_kv_tiles(dev, Hq, Hkv):
     want = ref.gqa_prefill(q.reshape(T, Hq, D), kv, r2t, rows, cu, rdy, Hq, Hkv, D)
     torch.cuda.synchronize()
     assert int(kernels().llb_attn_tc_status()) == 0, "a bounded wait inside the attention kernel ran out"
+    assert int(ops.gemm_status(dev).item()) == 0 and kernels().llb_attn_fa_status() == 0
     err = (got.float() - want.float()).abs().max().item()
     assert err < 2e-2, f"max abs err {err}"

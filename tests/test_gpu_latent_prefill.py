@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from lightllm_b200 import ops
 from lightllm_b200.ops import mla
 
 
@@ -44,6 +45,7 @@ def test_expanded_attention(new, ready, dv):
     want = _ref(q, kv, c[:, lat:], H, own, dv, cu, lens, ready, scale)
     # weights up to 2^-9 off (bf16 products), values of about 1, one rounding of the result
     assert (out.float() - want).abs().max().item() < 2e-2
+    assert int(ops.gemm_status("cuda:0").item()) == 0
 
 
 @pytest.mark.gpu
