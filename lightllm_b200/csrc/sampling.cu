@@ -183,7 +183,8 @@ sample_kernel(const T* __restrict__ logits, int64_t stride, int V, const float* 
   if (threadIdx.x == 0) {
     int id = pick.i == 0x7fffffff ? best.i : pick.i;
     out_ids[b] = id;
-    if (out_logprob) out_logprob[b] = ld_logit(row, id) * inv_t - xmax - logz;
+    // a row of NaN has no token: nothing to read at its index
+    if (out_logprob) out_logprob[b] = id < V ? ld_logit(row, id) * inv_t - xmax - logz : NAN;
   }
 }
 
@@ -337,7 +338,8 @@ sample_row_kernel(const T* __restrict__ logits, int64_t stride, int V, int slice
   if (rank == 0 && threadIdx.x == 0) {
     const int id = pick.i == 0x7fffffff ? best.i : pick.i;
     out_ids[b] = id;
-    if (out_logprob) out_logprob[b] = ld_logit(row, id) * inv_t - xmax - logz;
+    // a row of NaN has no token: nothing to read at its index
+    if (out_logprob) out_logprob[b] = id < V ? ld_logit(row, id) * inv_t - xmax - logz : NAN;
   }
 }
 

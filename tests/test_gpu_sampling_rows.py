@@ -73,3 +73,17 @@ def test_greedy(V, pad, dtype):
     assert torch.equal(ids, want)
     ref_lp = torch.log_softmax(x.double(), -1).gather(1, want[:, None])[:, 0]
     assert (lp.double() - ref_lp).abs().max().item() < 1e-4   # fp32 sums of up to 1e5 positive terms, fast exp and log
+
+
+@pytest.mark.parametrize("V", [100, 5000])
+def test_a_row_of_nan(V):
+    """A row without a single number has no token: the index says so, nothing is read there, and the other rows are drawn as they are alone."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(3, V, device="cuda", generator=g)
+    args = [torch.full((3,), t, device="cuda") for t in (0.8, 0.9)] + [torch.full((3,), 20, dtype=torch.int32, device="cuda")] + \
+        [torch.arange(3, device="cuda") + s for s in (5, 7)]
+    want, want_lp = ops.sample(x, *args)
+    x[1] = float("nan")
+    ids, lp = ops.sample(x, *args)
+    assert ids[1] == 0x7fffffff and lp[1].isnan()
+    assert torch.equal(ids[::2], want[::2]) and torch.equal(lp[::2], want_lp[::2])
