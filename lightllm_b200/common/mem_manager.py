@@ -402,8 +402,11 @@ class MLAMemoryManager(MemoryManager):
         return layer_num * (kv_lora_rank + rope_dim) * torch.empty((), dtype=dtype).element_size()
 
 
+PASS_RESERVE_BYTES = 6 << 30   # activations of a pass and CUDA graphs
+
+
 def profile_max_tokens(device: torch.device, bytes_per_token: int, mem_fraction: float = 0.9,
-                       reserve_bytes: int = 6 << 30) -> int:
+                       reserve_bytes: int = PASS_RESERVE_BYTES) -> int:
     """Tokens that fit in `mem_fraction` of the currently free device memory, leaving `reserve_bytes`
     for activations and CUDA graphs."""
     if device.type != "cuda":

@@ -28,7 +28,7 @@ import torch
 
 from .. import ops
 from ..common.infer_state import ShardedLogits, InferState, ModelInput, ModelOutput
-from ..common.mem_manager import MemoryManager, profile_max_tokens
+from ..common.mem_manager import PASS_RESERVE_BYTES, MemoryManager, profile_max_tokens
 from ..common.req_manager import ReqManager
 from ..ops import reference as ref
 from ..parallel import dist as pdist
@@ -434,9 +434,14 @@ class TransformerLM:
     def _kv_layer(self, i: int):
         return self.mem_manager.layer(self.kv_layer_offset + i)
 
+    def _pass_reserve_bytes(self) -> int:
+        """Memory that a pass of this model needs beyond PASS_RESERVE_BYTES."""
+        return 0
+
     def _init_mem(self, max_total_token_num, mem_fraction):
         if max_total_token_num is None:
-            max_total_token_num = profile_max_tokens(self.device, self.kv_bytes_per_token(), mem_fraction)
+            max_total_token_num = profile_max_tokens(self.device, self.kv_bytes_per_token(), mem_fraction,
+                                                     PASS_RESERVE_BYTES + self._pass_reserve_bytes())
             if self.ps.world_size > 1:
                 import torch.distributed as dist
 

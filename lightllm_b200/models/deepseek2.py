@@ -175,7 +175,6 @@ class DeepseekV2LM(TransformerLM):
         if self._can_expand():   # both halves as one K-major matrix: latent row -> [all heads' keys | all heads' values]
             n = (h1 - h0) * self.nope
             lw.w_kv = self._dev(torch.cat([kvb[:, : self.nope].reshape(n, -1), kvb[:, self.nope:].reshape(-1, self.kv_lora)]))
-            lw.w_uv = lw.w_kv[n:].view(h1 - h0, self.v_dim, self.kv_lora)
         else:
             lw.w_uv = self._dev(kvb[:, self.nope:])
         if self.fp8_compute and (h0 * self.v_dim) % 128 == 0:
@@ -247,7 +246,7 @@ class DeepseekV2LM(TransformerLM):
             return self._expanded_attention(lw, q, kv_layer, st, groups)
         q_lat = mla_ops.gemm_batched(q3[:, :, :nope], lw.w_uk)    # [T, hq, kvl]
         o_lat = self._mla_attend(i, lw, h, q_a if self.q_lora else None, q_lat, q3[:, :, nope:], kv_layer, st)
-        o = mla_ops.gemm_batched(o_lat, lw.w_uv)                  # [T, hq, v]
+        o = mla_ops.gemm_batched(o_lat, self._w_uv(lw))           # [T, hq, v]
         return o.reshape(T, hq * self.v_dim)
 
     def _can_expand(self) -> bool:
@@ -255,6 +254,20 @@ class DeepseekV2LM(TransformerLM):
         attention over all cached positions (sparse variants select in the latent space)."""
         return self.device.type == "cuda" and self.dtype == torch.bfloat16 and self.nope == 128 and self.rope_d == 64 and \
             self.v_dim in (64, 128) and self.sm_scale > 0 and type(self)._mla_attend is DeepseekV2LM._mla_attend
+
+    def _w_uv(self, lw):
+        """[hq, v, kv_lora].  Where w_kv holds it, a view made at each use: a second tensor over the same storage would come back from
+        a release of the weights as a copy."""
+        return lw.w_uv if lw.w_kv is None else lw.w_kv[self.hq * self.nope:].view(self.hq, self.v_dim, self.kv_lora)
+
+    def _pass_reserve_bytes(self) -> int:
+        """What a prompt pass in the expanded form holds beyond the latent queries and outputs of the other form: keys and values, and the
+        gathered latent rows they come from."""
+        if not self._can_expand():
+            return 0
+        rows = mla_ops.EXPANDED_BYTES // (self.hq * (self.nope + self.v_dim) * 2)
+        latent = 2 * int(self.batch_max_tokens) * self.hq * self.kv_lora * 2
+        return max(0, mla_ops.EXPANDED_BYTES + rows * (self.kv_lora + self.rope_d) * 2 - latent)
 
     def _expanded_groups(self, st):
         if not st.is_prefill or not self._can_expand():

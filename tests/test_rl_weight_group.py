@@ -116,3 +116,43 @@ def test_release_and_resume_weights_with_and_without_host_backup():
     rl_ops.resume_memory_occupation(loop, tags=("weights",))
     assert m.lm_head_w.shape == head_before.shape and float(m.lm_head_w.abs().sum()) == 0.0   # to be filled by a push
     assert (m.lm_head_w is m.embed_w) == tied
+
+
+def test_latent_weights_hold_their_bytes_over_release_and_resume(monkeypatch):
+    """Latent attention that forms keys and values per head keeps both halves of kv_b in one matrix: no second tensor over the same storage,
+    which a release and resume of the weights would bring back as a copy; and the KV pool leaves room for the expanded rows."""
+    from lightllm_b200.common import mem_manager
+    from lightllm_b200.models import base
+    from lightllm_b200.models.deepseek2 import DeepseekV2LM
+    from lightllm_b200.models.registry import get_model
+    from lightllm_b200.ops import mla
+
+    cfg = dict(model_type="deepseek_v3", hidden_size=64, intermediate_size=128, moe_intermediate_size=32, num_hidden_layers=2,
+               num_attention_heads=4, num_key_value_heads=4, n_routed_experts=4, n_shared_experts=1, num_experts_per_tok=2, n_group=1,
+               topk_group=1, first_k_dense_replace=1, q_lora_rank=32, kv_lora_rank=48, qk_nope_head_dim=16, qk_rope_head_dim=8,
+               v_head_dim=16, vocab_size=200, max_position_embeddings=256, routed_scaling_factor=2.5, norm_topk_prob=True, rms_norm_eps=1e-6)
+    reserves = []
+    monkeypatch.setattr(base, "profile_max_tokens", lambda dev, per, frac, reserve: reserves.append(reserve) or 512)
+
+    def model(expand):
+        monkeypatch.setattr(DeepseekV2LM, "_can_expand", lambda self: expand)
+        return get_model(cfg, pstate=pdist.ParallelState(device=torch.device("cpu")), data_type="float32", max_req_num=4,
+                         max_seq_length=128, disable_cudagraph=True, random_seed=3)
+
+    latent, m = model(False), model(True)
+    for a, b in zip(latent.layers, m.layers):
+        assert torch.equal(latent._w_uv(a), m._w_uv(b)) and torch.equal(a.w_uk, b.w_uk)
+    bytes_of = lambda: sum(t.untyped_storage().nbytes() for t in {id(t): t for _, _, t in rl_ops._weight_slots(m)}.values())  # noqa: E731
+    loop = SimpleNamespace(model=m, backend=SimpleNamespace(has_work=lambda: False, radix_cache=None), args=SimpleNamespace(enable_weight_cpu_backup=True))
+    before = bytes_of()
+    rl_ops.release_memory_occupation(loop, tags=("weights",))
+    rl_ops.resume_memory_occupation(loop, tags=("weights",))
+    assert bytes_of() == before
+    for a, b in zip(latent.layers, m.layers):
+        assert torch.equal(latent._w_uv(a), m._w_uv(b))
+    # 16384 tokens a pass: the expanded rows less the latent queries and outputs of that many tokens
+    rows = mla.EXPANDED_BYTES // (4 * 32 * 2)
+    assert reserves[0] == mem_manager.PASS_RESERVE_BYTES
+    assert reserves[1] - reserves[0] == mla.EXPANDED_BYTES + rows * 56 * 2 - 2 * m.batch_max_tokens * 4 * 48 * 2 > 0
+    del latent, m
+    pdist.destroy()
