@@ -213,13 +213,13 @@ class TiledWeight:
 _autotuner = None
 
 
-def _tuned_bn(M: int, N: int, K: int, epi: str) -> int:
+def _tuned_bn(M: int, N: int, K: int, epi: str, few: bool = False) -> int:
     global _autotuner
     if _autotuner is None:
         from ..utils import autotuner as _autotuner_mod
 
         _autotuner = _autotuner_mod
-    return _autotuner.gemm_lookup(M, N, K, epi)
+    return _autotuner.gemm_lookup(M, N, K, epi, few)
 
 
 # Up to this many tokens a plain weight goes through csrc/gemm_stream.cu (weights as the MMA's M side).
@@ -228,10 +228,14 @@ _STREAM_EPIS = ("store", "residual", "gated_silu", "f32", "gated_gelu", "relu2")
 
 
 def _stream_rule(M: int, N: int, K: int, epi: str, bias) -> bool:
-    """Up to 64 tokens always.  With more of them a CTA stages as many token bytes as weight bytes, and the 256-column kernels are
-    ahead (B200, us per call in a chain, here / there: [4096, 14336] 42 / 35, [6144, 4096] 22 / 18, and [128256, 4096] 210 / 196,
-    whose tiles read the tokens once per wave), except where those leave SMs idle: a weight whose 128-row tiles fill one and a half to
-    two CTAs per SM without shares of K ([28672, 4096] 51 / 93), or a small one ([5120, 2048] 12 / 17, [2048, 4096] 14 / 17)."""
+    """Up to 64 tokens always; a variant of the tile kernels that a table found faster all the same goes first (see `gemm`).  B200, us for
+    norm + GEMM in a chain, here / the best of the tile kernels: 1 token [6144, 4096] 16.1 / 25.9, [28672, 4096] 43 / 78, [4096, 14336]
+    31 / 52; 64 tokens 20.2 / 19.5, 48 / 92, 36.1 / 35.3, [16032, 4096] 35.3 / 32.0 (the widest gap of 43 shapes), [1536, 4096] 11.5 / 14.1,
+    [4096, 3584] 14.3 / 15.4, [57344, 8192] 161 / 184.
+    With 65 to 128 tokens a CTA stages as many token bytes as weight bytes, and the 256-column kernels are ahead (128 tokens: [4096, 14336]
+    42.7 / 36.1, [6144, 4096] 23.8 / 19.7, [128256, 4096] 214 / 200), except where those leave SMs idle: a weight whose 128-row tiles make
+    one to two CTAs per SM without shares of K (128 tokens: [20480, 4096] 45 / 51, [24576, 2048] 30.5 / 71, [28672, 4096] 53 / 93, [28672,
+    8192] 94 / 135, [36864, 4096] 62.7 / 64.0), or a small one ([2048, 4096] 14 / 17, [5120, 2048] 12 / 17, [3072, 4096] 16.1 / 15.9)."""
     if not (0 < M <= STREAM_MAX_M and N >= 1024 and K >= 1024 and N % 8 == 0 and epi in _STREAM_EPIS):
         return False
     if bias is not None and epi.startswith("gated"):
@@ -283,9 +287,10 @@ def gemm(a, w, epi: str = "store", residual=None, bias=None, out=None, bn: int =
     N = w.shape[0]
     if stream_k == 0 and not isinstance(w, TiledWeight) and (4000 <= bn < 4100 or bn == 0 and _stream_rule(M, N, K, epi, bias)) and \
             not kernels().llb_gemm_push_armed():   # a push set up for this call: the tile kernels make it
-        if bn == 0:   # a stored variant of this kernel is a number of K shares; other variants were tuned before it was there
-            bn = _tuned_bn(M, N, K, epi) if bias is None else 0
-        return _gemm_stream(a, w, epi, residual, bias, out, bn - 4000 if 4000 <= bn < 4100 else 0, w_ready)
+        if bn == 0 and bias is None:   # a number of K shares, or a variant of the tile kernels that was timed against this one
+            bn = _tuned_bn(M, N, K, epi, few=True)
+        if bn == 0 or 4000 <= bn < 4100:
+            return _gemm_stream(a, w, epi, residual, bias, out, max(bn - 4000, 0), w_ready)
     return _gemm_tiles(a, w, epi, residual, bias, out, bn, stream_k)
 
 

@@ -163,7 +163,8 @@ GEMM_KERNEL = "gemm_bf16"
 # `bn` selectors understood by ops.gemm: 0 automatic plan, 64 / 128 / 256 one-CTA tiles, 512 CTA-pair tiles,
 # 1000 + 10 * accumulators + splits cluster kernel (+ 100: 128-column tiles), 2000 + splits one-CTA tiles and
 # 3000 + splits CTA-pair tiles with K split through the L2 workspace (x000: as many splits as fit), 4000 + splits the few-token
-# kernel (the only variants looked at where `ops._stream_rule` holds)
+# kernel.  Where `ops._stream_rule` holds, 0 is that kernel with its own plan, and a stored variant counts if that kernel was timed with
+# it ("few": 1); entries without the mark hold the best of the tile kernels, which other callers use (a push to tensor-parallel peers).
 GEMM_CANDIDATES = [{"bn": b} for b in (0, 64, 128, 256, 512, 1011, 1012, 1014, 1021, 1111, 1112,
                                        2000, 2002, 2004, 3000, 3001, 3002, 3004, 4001, 4002, 4003, 4004, 4006, 4008)]
 
@@ -172,10 +173,16 @@ def gemm_static_key(N: int, K: int, epi: str) -> str:
     return f"N={N},K={K},epi={epi}"
 
 
-def gemm_lookup(M: int, N: int, K: int, epi: str) -> int:
-    """The tuned `bn` selector for this problem, 0 (the built-in plan) when nothing is stored."""
-    cfg = store().lookup(GEMM_KERNEL, gemm_static_key(N, K, epi), M)
-    return int(cfg["bn"]) if cfg else 0
+_timing = False   # while variants are timed, 0 is the built-in plan, whatever is stored
+
+
+def gemm_lookup(M: int, N: int, K: int, epi: str, few: bool = False) -> int:
+    """The tuned `bn` selector for this problem, 0 (the built-in plan) when nothing is stored.  few: only of entries that were timed
+    against the few-token kernel; else the best of the others."""
+    cfg = None if _timing else store().lookup(GEMM_KERNEL, gemm_static_key(N, K, epi), M)
+    if not cfg or few and not cfg.get("few"):
+        return 0
+    return int(cfg["bn"] if few else cfg.get("tile", cfg["bn"]))
 
 
 def tune_gemm(M: int, N: int, K: int, epi: str = "store", group=None, reps: int = 16, save: bool = True) -> dict:
@@ -196,18 +203,25 @@ def tune_gemm(M: int, N: int, K: int, epi: str = "store", group=None, reps: int 
     del ref
 
     def bench(c):
-        fn = lambda i: ops.gemm(xs[i % copies], ws[i % copies], epi=epi, residual=res, bn=c["bn"])  # noqa: E731
+        fn = lambda i: ops.gemm(xs[i % copies], ws[i % copies], epi=epi, residual=res, bn=c["bn"], w_ready=True)  # noqa: E731
         fn(0)  # unsupported variants raise here
         torch.cuda.synchronize()
         return timeit_graph(fn, flush, n=9, reps=reps)
 
-    best, scored = tune(GEMM_CANDIDATES, bench, group)
+    global _timing
+    _timing = True
+    try:
+        best, scored = tune(GEMM_CANDIDATES, bench, group)
+    finally:
+        _timing = False
     t_best = scored[0][0]
     t_auto = next((t for t, c in scored if c["bn"] == 0), float("inf"))
     if t_auto <= t_best * 1.03:  # within measurement noise of the built-in plan: keep the plan
         best, t_best = {"bn": 0}, t_auto
-    store().store(GEMM_KERNEL, gemm_static_key(N, K, epi), M, {"bn": best["bn"], "us": round(t_best * 1e3, 2)},
-                  save=save)
+    cfg = {"bn": best["bn"], "us": round(t_best * 1e3, 2), "few": 1}
+    if ops._stream_rule(M, N, K, epi, None):   # the best one for callers that the few-token kernel does not serve
+        cfg["tile"] = next((c["bn"] for t, c in scored if 0 < c["bn"] < 4000 and t < float("inf")), 0)
+    store().store(GEMM_KERNEL, gemm_static_key(N, K, epi), M, cfg, save=save)
     return best
 
 

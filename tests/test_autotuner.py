@@ -67,3 +67,53 @@ def test_candidates_are_split_across_ranks(tmp_path):
     a, b = torch.load(tmp_path / "r0.pt"), torch.load(tmp_path / "r1.pt")
     assert a["best"] == b["best"] == {"bn": 7} and a["n"] == b["n"] == 12
     assert sorted(a["seen"] + b["seen"]) == list(range(12)) and not set(a["seen"]) & set(b["seen"])
+
+
+def test_few_token_gemm_and_stored_variants(tmp_path, monkeypatch):
+    """Few tokens: a stored variant of the tile kernels counts if it was timed against the few-token kernel; a push to tensor-parallel peers,
+    which only the tile kernels make, gets the best of those."""
+    from lightllm_b200 import ops
+
+    N, K, armed, calls = 4096, 4096, [0], []
+
+    class Fake:
+        def llb_gemm_push_armed(self):
+            return armed[0]
+
+        def llb_gemm_stream(self, *a):
+            calls.append(("few", a[12].value))
+            return 0
+
+        def llb_gemm_bf16(self, *a):
+            calls.append(("tile", a[12].value))
+            return 0
+
+    word = torch.zeros(1, dtype=torch.int32)
+    for name, value in (("kernels", Fake), ("gemm_status", lambda d: word), ("stream", lambda: None), ("_is_cuda", lambda t: True),
+                        ("_stream_k_scratch", lambda d: (word.float(), word))):
+        monkeypatch.setattr(ops, name, value)
+    monkeypatch.setattr(at, "PKG_DIR", tmp_path / "pkg")
+    st = at.KernelConfigStore(device="devX", user_dir=str(tmp_path / "user"))
+    key = at.gemm_static_key(N, K, "store")
+    for M, cfg in ((1, {"bn": 2000}), (16, {"bn": 2002, "few": 1}), (32, {"bn": 4003, "few": 1, "tile": 2004}), (64, {"bn": 0, "few": 1, "tile": 1012})):
+        st.store("gemm_bf16", key, M, cfg, save=False)
+    at.reset_store(st)
+    w = torch.zeros(N, K, dtype=torch.bfloat16)
+    try:
+        def route(M, push=0):
+            armed[0] = push
+            ops.gemm(torch.zeros(M, K, dtype=torch.bfloat16), w)
+            return calls.pop()
+
+        assert [route(M) for M in (1, 16, 32, 64)] == [("few", 0), ("tile", 2002), ("few", 3), ("few", 0)]
+        assert [route(M, push=2) for M in (1, 16, 32, 64)] == [("tile", 2000), ("tile", 2002), ("tile", 2004), ("tile", 1012)]
+    finally:
+        at.reset_store(None)
+
+
+def test_shipped_table_keeps_the_variants_of_few_tokens():
+    """A row-parallel projection of a tensor-parallel rank is pushed to its peers by the tile kernels with 1 to 8 tokens too: the variants
+    tuned at those sizes are there, not the nearest one of 128 tokens."""
+    table = json.loads((at.PKG_DIR / "NVIDIA_B200" / "gemm_bf16.json").read_text())
+    for N, K in ((4096, 1024), (4096, 1792), (4096, 2048), (4096, 3584), (4096, 7168), (8192, 1024), (8192, 3584)):
+        assert {"1", "8", "16", "32", "64", "128"} <= set(table[f"N={N},K={K},epi=store"])
