@@ -1,8 +1,8 @@
 // Prompt attention on tcgen05 with scores, weights and outputs in tensor memory: causal, varlen, aware of cached positions.
 //
 //   paged    K/V rows of the token-granular pool, fetched by TMA gathers through the slot table (head size 128)
-//   expanded K/V rows of dense matrices formed for the pass (latent attention: key size 192, value size 128 or 64; the last columns
-//            of a head's keys may be shared by all heads, see llb_latent_prefill_fa)
+//   expanded K/V rows of dense matrices formed for the pass (latent attention: key size 192, value size 128 or 64; the last 64 columns
+//            of the keys are shared by all heads, see llb_latent_prefill_fa)
 //
 // A CTA works on two 128-row query tiles against the same keys: two query heads of one KV head where their number is even (paged), else
 // 256 consecutive tokens of a head.  Per tile of BN keys and query tile t:
@@ -30,6 +30,7 @@ LLB_DEBUG_BOUNDS_STORAGE(attention_fa)
 namespace {
 
 constexpr int BM = 128;
+constexpr int OWN = 128;          // expanded: key columns of a head's own; the others are shared by all heads
 constexpr int THREADS = 12 * 32;  // warp 0: Q and K/V loads (paged: with warps 2, 3), warp 1: MMA, warps 4..7 / 8..11: softmax of query
                                   // tile 0 / 1
 constexpr float kLog2e = 1.4426950408889634f;
@@ -59,7 +60,7 @@ struct Params {
   int64_t r2t_stride;
   // expanded
   const int *cu_kv, *kv_start;
-  int own, shared_col;
+  int shared_col;
 };
 
 __device__ __forceinline__ float ex2_fast(float x) {  // 2^x, one MUFU instruction (x = -inf gives 0)
@@ -193,14 +194,14 @@ prefill_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         mbar_expect_tx(k_full(ks), L::K_BYTES);
 #pragma unroll
         for (int c = 0; c < DK / 64; ++c) {
-          const bool mine = c * 64 < p.own;
+          const bool mine = c * 64 < OWN;
           tma_load_2d(smem_base + L::OFF_K + ks * L::K_BYTES + c * BN * 128, mine ? &tmKV : &tmShared, k_full(ks),
-                      mine ? y * p.own + c * 64 : p.shared_col + c * 64 - p.own, row0 + j * BN);
+                      mine ? y * OWN + c * 64 : p.shared_col + c * 64 - OWN, row0 + j * BN);
         }
         if (!mbar_wait(v_empty(vs), ((j / VS) & 1) ^ 1, abort_flag, status, 72)) break;
         mbar_expect_tx(v_full(vs), L::V_BYTES);
         const uint32_t v = smem_base + L::OFF_V + vs * L::V_BYTES;
-        const int v_col = p.Hq * p.own + y * DV;
+        const int v_col = p.Hq * OWN + y * DV;
         if ((j + 1) * BN <= rows) {
 #pragma unroll
           for (int c = 0; c < DV / 64; ++c) tma_load_2d(v + c * BN * 128, &tmKV, v_full(vs), v_col + c * 64, row0 + j * BN);
@@ -421,33 +422,30 @@ LLB_EXPORT int llb_gqa_prefill_fa(const void* q, int64_t q_stride, int T, const 
   return launch_fa<128, 128, 128, true, false>(tq, tkv, tkv, tkv, p, B, max_q_len, st);
 }
 
-// q [T, >= H * 192] bf16 (row pitch q_stride), kv [kv_rows, H * own | H * dv] (pitch kv_stride), out [T, >= H * dv].  Request b's
-// keys are rows cu_kv[b] .., position kv_start[b] first.  own 192, or 128: the last 64 columns of every head's keys are then columns
-// shared_col .. of `shared` [kv_rows, >= shared_col + 64] (pitch shared_stride).
+// q [T, >= H * 192] bf16 (row pitch q_stride), kv [kv_rows, H * 128 | H * dv] (pitch kv_stride), out [T, >= H * dv].  Request b's
+// keys are rows cu_kv[b] .., position kv_start[b] first; the last 64 columns of every head's keys are columns shared_col .. of `shared`
+// [kv_rows, >= shared_col + 64] (pitch shared_stride).
 LLB_EXPORT int llb_latent_prefill_fa(const void* q, int64_t q_stride, const void* kv, int64_t kv_stride, int kv_rows,
-                                     const void* shared, int64_t shared_stride, int shared_col, int own, const int* cu_q,
+                                     const void* shared, int64_t shared_stride, int shared_col, const int* cu_q,
                                      const int* cu_kv, const int* kv_start, const int* b_ready_len, void* out, int64_t out_stride,
                                      int B, int T, int max_q_len, int H, int dv, float sm_scale, int* status, cudaStream_t st) {
   if (B <= 0 || max_q_len <= 0 || T <= 0) return LLB_OK;
   if (!(sm_scale > 0.f) || status == nullptr || H <= 0 || kv_rows <= 0 || (out_stride % 8) || ((uintptr_t)out & 15)) return LLB_ERR_BAD_ARG;
-  if (B > 65535 || cdiv(max_q_len, BM) > 65535 || (dv != 64 && dv != 128) || (own != 128 && own != 192)) return LLB_ERR_UNSUPPORTED;
-  if (own == 128 && (shared == nullptr || shared_col < 0 || (shared_col % 8))) return LLB_ERR_BAD_ARG;
+  if (B > 65535 || cdiv(max_q_len, BM) > 65535 || (dv != 64 && dv != 128)) return LLB_ERR_UNSUPPORTED;
+  if (shared == nullptr || shared_col < 0 || (shared_col % 8)) return LLB_ERR_BAD_ARG;
   CUtensorMap tq, tkv, ts, trow;
   int rc = make_tmap_2d(&tq, q, 2, (uint64_t)T, (uint64_t)H * 192, (uint64_t)q_stride, BM, 64);
   if (rc) return rc;
-  rc = make_tmap_2d(&tkv, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (own + dv), (uint64_t)kv_stride, 64, 64);
+  rc = make_tmap_2d(&tkv, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (OWN + dv), (uint64_t)kv_stride, 64, 64);
   if (rc) return rc;
-  rc = make_tmap_2d(&trow, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (own + dv), (uint64_t)kv_stride, 1, 64);
+  rc = make_tmap_2d(&trow, kv, 2, (uint64_t)kv_rows, (uint64_t)H * (OWN + dv), (uint64_t)kv_stride, 1, 64);
   if (rc) return rc;
-  ts = tkv;
-  if (own == 128) {
-    rc = make_tmap_2d(&ts, shared, 2, (uint64_t)kv_rows, (uint64_t)shared_col + 64, (uint64_t)shared_stride, 64, 64);
-    if (rc) return rc;
-  }
+  rc = make_tmap_2d(&ts, shared, 2, (uint64_t)kv_rows, (uint64_t)shared_col + 64, (uint64_t)shared_stride, 64, 64);
+  if (rc) return rc;
   Params p;
   memset(&p, 0, sizeof(p));
   p.status = status, p.cu_q = cu_q, p.b_ready_len = b_ready_len, p.out = (bf16*)out, p.out_stride = out_stride, p.scale_log2 = sm_scale * kLog2e;
-  p.Hq = p.Hkv = H, p.n_slots = kv_rows, p.cu_kv = cu_kv, p.kv_start = kv_start, p.own = own, p.shared_col = shared_col;
+  p.Hq = p.Hkv = H, p.n_slots = kv_rows, p.cu_kv = cu_kv, p.kv_start = kv_start, p.shared_col = shared_col;
   return dv == 64 ? launch_fa<192, 64, 64, false, true>(tq, tkv, ts, trow, p, B, max_q_len, st)
                   : launch_fa<192, 128, 64, false, true>(tq, tkv, ts, trow, p, B, max_q_len, st);
 }

@@ -551,10 +551,6 @@ LLB_EXPORT int llb_quant_fp8_group128_rows(const void* x, int64_t ldx, void* q, 
                              scale_ld, M, K, kg, pair);
   return e == cudaSuccess ? LLB_OK : (int)e;
 }
-LLB_EXPORT int llb_quant_fp8_group128(const void* x, int64_t ldx, void* q, int64_t ldq, float* scale,
-                                      int64_t scale_ld, int M, int K, cudaStream_t st) {
-  return llb_quant_fp8_group128_rows(x, ldx, q, ldq, scale, scale_ld, M, K, nullptr, st);
-}
 
 namespace {
 template <int TBN>

@@ -558,10 +558,6 @@ LLB_EXPORT int llb_moe_gather_rows(void* a_sorted, const void* x, const int* sor
   LLB_LAUNCH_CHECK();
   return LLB_OK;
 }
-LLB_EXPORT int llb_moe_gather(void* a_sorted, const void* x, const int* sorted_pair, const int* total_rows, int k,
-                              int H, int64_t x_stride, int max_rows, cudaStream_t st) {
-  return llb_moe_gather_rows(a_sorted, x, sorted_pair, total_rows, k, H, x_stride, max_rows, 1, st);
-}
 
 LLB_EXPORT int llb_moe_combine(void* out, const void* y, const int* pair_row, const float* weights, int T, int k, int H,
                                int accumulate, cudaStream_t st) {

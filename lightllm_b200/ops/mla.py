@@ -286,14 +286,14 @@ def window_prefill(q, kv, H: int, dk: int, dv: int, cu_q, b_ready_len, kr: KeyRa
 
 def latent_prefill(q, kv, c, col: int, own: int, H: int, dk: int, dv: int, cu_q, b_ready_len, kr: KeyRange, max_q_len: int, scale,
                    out):
-    """Expanded form without a window (`csrc/attention_fa.cu`), key size 192: q [T, >= H * dk] (row stride free), kv [rows, H * own |
-    H * dv], own 192, or 128: the last 64 columns of every head's keys are the columns from `col` on of c [rows, >= col + 64].  out
-    [T, H * dv] (only the requests of cu_q are written)."""
-    assert q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16 and c.dtype == torch.bfloat16 and dk == 192
+    """Expanded form without a window (`csrc/attention_fa.cu`), key size dk 192: q [T, >= H * dk] (row stride free), kv [rows, H * own |
+    H * dv] with own 128; the last 64 columns of every head's keys are the columns from `col` on of c [rows, >= col + 64].  out [T, H * dv]
+    (only the requests of cu_q are written)."""
+    assert q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16 and c.dtype == torch.bfloat16 and dk == 192 and own == 128
     assert q.stride(1) == 1 and kv.is_contiguous() and c.stride(1) == 1 and out.stride(1) == 1 and cu_q.dtype == torch.int32
     assert kv.shape == (kr.rows, H * (own + dv)) and c.shape[0] == kr.rows and c.shape[1] >= col + dk - own
     check(kernels().llb_latent_prefill_fa(ptr(q), i64(q.stride(0)), ptr(kv), i64(kv.stride(0)), c_int(kr.rows), ptr(c),
-                                          i64(c.stride(0)), c_int(col), c_int(own), ptr(cu_q), ptr(kr.cu_kv), ptr(kr.kv_start),
+                                          i64(c.stride(0)), c_int(col), ptr(cu_q), ptr(kr.cu_kv), ptr(kr.kv_start),
                                           ptr(b_ready_len), ptr(out), i64(out.stride(0)), c_int(cu_q.shape[0] - 1),
                                           c_int(q.shape[0]), c_int(max_q_len), c_int(H), c_int(dv), f32(scale),
                                           ptr(gemm_status(q.device)), stream()),
