@@ -700,8 +700,8 @@ LLB_EXPORT int llb_window_gqa_decode(const void* q, int64_t q_stride, const void
   return LLB_ERR_UNSUPPORTED;
 }
 
-// tcgen05 kernel for head size 128 (attention_tc.cu), for rows that the TMA kernel (llb_gqa_prefill_fa, attention_fa.cu; chosen by the
-// caller) cannot read; LLB_ATTN_TC=0 keeps the mma.sync kernel below
+// One-tile tcgen05 kernel for head size 128 (attention_tc.cu).  Callers take llb_gqa_prefill_fa (attention_fa.cu) ahead of this entry for all
+// rows that either kernel can read, unless LLB_ATTN_FA=0 asks for this one; LLB_ATTN_TC=0 keeps the mma.sync kernel below
 LLB_EXPORT int llb_gqa_prefill_tc(const void* q, int64_t q_stride, const void* kv_layer, const int* req_to_token,
                                   int64_t r2t_stride, const int* b_req_idx, const int* cu_q, const int* b_ready_len,
                                   void* out, int64_t out_stride, int B, int max_q_len, int Hq, int Hkv, float sm_scale,

@@ -21,7 +21,10 @@ DTYPE_CODES = {torch.float32: 0, torch.bfloat16: 1}   # kernels that exist in bo
 
 import os as _os
 
-_ATTN_TC = _os.environ.get("LLB_ATTN_TC", "1") != "0"   # 0: prompt attention on the mma.sync kernel, for comparison
+# Prompt attention of head size 128, for comparison: LLB_ATTN_FA=0 on the one-tile tcgen05 kernel (csrc/attention_tc.cu), LLB_ATTN_TC=0 on
+# the mma.sync kernel (csrc/attention.cu)
+_ATTN_TC = _os.environ.get("LLB_ATTN_TC", "1")[:1] != "0"
+_ATTN_FA = _ATTN_TC and _os.environ.get("LLB_ATTN_FA", "1")[:1] != "0"
 _GEMM_DEBUG_TORCH = _os.environ.get("LLB_GEMM_DEBUG_TORCH", "0") == "1"
 
 # launch counter: the number of kernels of this package launched (claimed in bench output)
@@ -464,7 +467,7 @@ def gqa_prefill(q, kv_layer, req_to_token, b_req_idx, cu_q, b_ready_len, Hq, Hkv
     scale = sm_scale if sm_scale is not None else 1.0 / math.sqrt(D)
     if out is None:
         out = torch.empty((T, Hq, D), dtype=q.dtype, device=q.device)
-    if D == 128 and _ATTN_TC and scale > 0 and T > 0 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and \
+    if D == 128 and _ATTN_FA and scale > 0 and T > 0 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and \
             out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and kv_layer.data_ptr() % 16 == 0:
         check(kernels().llb_gqa_prefill_fa(ptr(q), i64(q.stride(0)), c_int(T), ptr(kv_layer), c_int(kv_layer.shape[0]),
                                            ptr(req_to_token), i64(req_to_token.stride(0)), ptr(b_req_idx), ptr(cu_q),

@@ -50,6 +50,14 @@ def test_matches_fp32(new, ready, Hq, Hkv):
     assert (got - want).abs().max().item() < 2e-2
 
 
+def test_one_tile_kernel(monkeypatch):
+    """The kernel that LLB_ATTN_FA=0 selects."""
+    monkeypatch.setattr(ops, "_ATTN_FA", False)
+    got, want = _run([129, 1, 300], [0, 700, 127], 6, 2, pad=64)
+    assert kernels().llb_attn_tc_status() == 0
+    assert (got - want).abs().max().item() < 2e-2   # as above
+
+
 @pytest.mark.parametrize("grow", [1.0, 30.0])
 def test_moving_maximum(grow):
     got, want = _run([300, 128], [500, 0], 8, 2, scale=2.0, grow=grow)
