@@ -8,10 +8,11 @@
 // 256 consecutive tokens of a head.  Per tile of BN keys and query tile t:
 //   S_t  = Q_t . K^T     into tensor memory
 //   P_t  = exp2(S_t - m) one thread per row reads its scores, and writes the weights as bf16 over them in tensor memory (expanded form:
-//          as the sum of two bf16 values, which makes up for the rounding of the expanded keys and values)
+//          as the sum of two bf16 values, which makes up for the rounding of the expanded keys and values up to scores of spread 2.5)
 //   O_t += P_t . V       A operand from tensor memory, accumulated there over all key tiles
-// One thread issues all MMAs in the order  P0.V, Q0.K', P1.V, Q1.K'  so that the tensor core works on one query tile while the
-// softmax warps work on the other.  O is rescaled, read-multiply-write, when a row's maximum has grown: at once where the weights are
+// One thread issues all MMAs in the order  P0.V, Q0.K', P1.V, Q1.K'  so that the tensor core works on one query tile while the softmax
+// warps work on the other.  (This schedule, the weights as tensor-memory operand and the rescaling only after the maximum grew by 2^8 were
+// published with FlashAttention-4, Dao and others, 2025.)  O is rescaled, read-multiply-write, when a row's maximum has grown: at once where the weights are
 // single bf16 values, so that the weight of the largest key is exactly 1 (with a slack of 2^8 it is rounded like the others, and the error
 // against 64 bits grew from 0.0018 to 0.0023 for 1000 keys with scores of spread 2.5); by more than 2^8 where they are the sum of two.
 //

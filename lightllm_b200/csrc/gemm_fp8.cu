@@ -15,8 +15,8 @@
 // MMAs (2 TBN cycles), the operands' way from L2 (16 KB + TBN x 128 bytes) and the scaled sums, so
 //   * TBN = 256 where the tiles fill the GPU: 48 KB from L2 per group of 512 MMA cycles instead of 32 KB per 256
 //   * the scales of the next group are loaded while the current one is summed (they cost an L2 latency per group before)
-//   * two threads per row: half the sums and tensor-memory reads per warp  Grouped (MoE) mode: M-block i
-// multiplies with expert mblock_expert[i] of the stacked weights [E * N, K]; -1 skips the block.
+//   * two threads per row: half the sums and tensor-memory reads per warp
+// Grouped (MoE) mode: M-block i multiplies with expert mblock_expert[i] of the stacked weights [E * N, K]; -1 skips the block.
 #include "sm100_ptx.cuh"
 
 #include <cuda_fp8.h>

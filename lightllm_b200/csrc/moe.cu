@@ -538,6 +538,8 @@ LLB_EXPORT int llb_moe_align(const int* ids, int n_pairs, int e0, int E_local, i
                              int* pair_row, int* mblock_expert, int* expert_off, int* total_rows, cudaStream_t st) {
   if (E_local > 2048 || m_pad % 128 != 0) return LLB_ERR_UNSUPPORTED;
   int smem = (3 * E_local + 1) * sizeof(int);
+  // B200, us, one CTA / cluster: 4096 pairs of 8 experts 5.6 / 4.6, of 128 11.3 / 5.4, of 256 16.1 / 5.6; 65536 of 128 58.9 / 12.3.  Fewer
+  // pairs, decode steps, were not timed on the cluster.
   if (n_pairs >= 4096)
     moe_align_cluster_kernel<<<kAlignCtas, 1024, smem, st>>>(ids, n_pairs, e0, E_local, m_pad, sorted_pair, pair_row, mblock_expert,
                                                              expert_off, total_rows);

@@ -136,8 +136,10 @@ STREAM_MAX_M = 128
 
 def _stream_rule(M: int, N: int) -> bool:
     """The few-token kernel (csrc/gemm_stream.cu).  Above 64 tokens it reads every weight tile twice, which pays only for narrow
-    outputs, whose tiles would leave SMs idle otherwise (B200, us, here / there: 128 tokens [4096, 7168] 21 / 29, [8192, 8192] 39 / 35,
-    [57344, 8192] 188 / 104; 64 tokens [8192, 28672] 69 / 107, [8192, 8192] 23 / 34, [57344, 8192] 99 / 100)."""
+    outputs, whose tiles would leave SMs idle otherwise (B200, us with the quantisation, here / there: 128 tokens [1536, 7168] 14 / 27,
+    [4096, 7168] 22 / 27, [7168, 2048] 18 / 15, [8192, 8192] 40 / 33, [57344, 8192] 192 / 106).  64 tokens: [4096, 7168] 16 / 27, [8192, 28672]
+    75 / 103, [8192, 8192] 25 / 32, [57344, 8192] 104 / 103, [36864, 7168] 54 / 55; behind from 48 on for [24576, 1536] 17 / 15 and
+    [10240, 8192] 39 / 31, whose shares of K leave SMs idle, at the 20 and 38 of the kernels of before.  1 token: 1.25 to 2.2 times as fast."""
     return M <= (STREAM_MAX_M if N <= 4096 else min(64, STREAM_MAX_M))
 
 

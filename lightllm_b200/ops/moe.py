@@ -187,7 +187,10 @@ def gather_rows(x, lay: MoeLayout, zero_pad: bool = True):
     return a
 
 
-FEW_TOKENS = 128   # a decode step: every expert has at most one 128-row block
+# A decode step: every expert has at most one 128-row block.  B200, us for both GEMMs and what is around them, few-token form / padded blocks:
+# 128 experts of 768 and 8 choices 33 / 70 (1 token), 234 / 306 (64), 234 / 307 (128); 8 of 14336 and 2 choices 129 / 218, 458 / 522,
+# 483 / 593; fp8, 64 of 2048 and 8 choices 93 / 128, 504 / 736, 610 / 739 (its weights are read twice above 64 tokens)
+FEW_TOKENS = 128
 
 
 def _few_tokens_experts(x, w13, w2, lay, act):
