@@ -233,8 +233,8 @@ _STREAM_EPIS = ("store", "residual", "gated_silu", "f32", "gated_gelu", "relu2")
 def _stream_rule(M: int, N: int, K: int, epi: str, bias) -> bool:
     """Up to 64 tokens always; a variant of the tile kernels that a table found faster all the same goes first (see `gemm`).  B200, us for
     norm + GEMM in a chain, here / the best of the tile kernels: 1 token [6144, 4096] 16.1 / 25.9, [28672, 4096] 43 / 78, [4096, 14336]
-    31 / 52; 64 tokens 20.2 / 19.5 (17.7 with the table's 4 shares), 48 / 92, 36.1 / 35.3, [16032, 4096] 36.1 / 32.8 (the widest gap of 43
-    shapes; 30.0 with the table's 2 shares), [1536, 4096] 11.5 / 14.1, [4096, 3584] 14.3 / 15.4, [57344, 8192] 161 / 184.
+    31 / 52; 64 tokens 20.2 / 19.5 (in the table), 48 / 92, 36.1 / 35.3, [16032, 4096] 36.1 / 32.8 (the widest gap of 43 shapes; in the table),
+    [1536, 4096] 11.5 / 14.1, [4096, 3584] 14.3 / 15.4, [57344, 8192] 161 / 184.
     With 65 to 128 tokens a CTA stages as many token bytes as weight bytes, and the 256-column kernels are ahead (128 tokens: [4096, 14336]
     42.7 / 36.1, [6144, 4096] 23.8 / 19.7, [128256, 4096] 214 / 200), except where those leave SMs idle: a weight whose 128-row tiles make
     one to two CTAs per SM without shares of K (128 tokens: [20480, 4096] 45 / 51, [24576, 2048] 30.5 / 71, [28672, 4096] 53 / 93, [28672,
